@@ -316,3 +316,136 @@ def tolerance(case):
     if kind == "step":
         return {"rel": 2.4e-2, "max": 0.15}
     return {"rel": 1.2e-2, "max": 0.06}
+
+
+# ---- the same results in 64 bits, in plain torch --------------------------------------------------------------------
+
+def _f16_at(b):
+    """Little-endian fp16 bytes [..., 2] -> fp64 [...]."""
+    return b.contiguous().view(torch.float16).squeeze(-1).double()
+
+
+def _hadamard(v):
+    """Orthonormal Sylvester-Hadamard transform of every run of 128 along the last dimension."""
+    shape = v.shape
+    h = torch.ones(1, 1, dtype=torch.float64, device=v.device)
+    for _ in range(7):
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    return (v.reshape(-1, 128) @ (h / math.sqrt(128.0))).reshape(shape)
+
+
+def _dequantize(fmt, blocks, n, k):
+    """fp64 [n][k] weights of the packed blocks."""
+    if fmt == "tq3":
+        tiles = blocks[:n * k * 3 // 8].reshape(n // 16, k // 16, 96).to(torch.int64)
+        tiles = torch.nn.functional.pad(tiles, (0, 3))
+        bit = 3 * torch.arange(256, device=blocks.device)
+        window = tiles[..., bit // 8] | (tiles[..., bit // 8 + 1] << 8) | (tiles[..., bit // 8 + 2] << 16)
+        h = (((window >> (bit % 8)) & 0xffff) * 2654435761) & 0xffffffff
+        q = (sum((h >> s) & 255 for s in (0, 8, 16, 24)) - 510).double() / 147.8
+        q = q.reshape(n // 16, k // 16, 16, 16).transpose(1, 2).reshape(n, k)
+        scale = _f16_at(blocks[n * k * 3 // 8:n * k * 3 // 8 + 2 * n].reshape(n, 2))
+        signs = blocks[n * k * 3 // 8 + 2 * n:].reshape(-1, 1).to(torch.int64) >> torch.arange(8, device=blocks.device) & 1
+        return scale[:, None] * _hadamard(_hadamard(q).t()).t() * (1.0 - 2.0 * signs.reshape(k).double())
+    if fmt == "q8_0":
+        b = blocks.reshape(n, k // 32, 34)
+        return (_f16_at(b[..., :2])[..., None] * b[..., 2:].contiguous().view(torch.int8).double()).reshape(n, k)
+    if fmt == "q4_k":
+        b = blocks.reshape(n, k // 256, 144)
+        s = b[..., 4:16].to(torch.int64)
+        sc = torch.cat([s[..., 0:4] & 63, (s[..., 8:12] & 15) | ((s[..., 0:4] >> 6) << 4)], -1).double()
+        mn = torch.cat([s[..., 4:8] & 63, (s[..., 8:12] >> 4) | ((s[..., 4:8] >> 6) << 4)], -1).double()
+        qs = b[..., 16:].reshape(n, k // 256, 4, 32)
+        q = torch.stack([qs & 15, qs >> 4], dim=3).reshape(n, k // 256, 8, 32).double()
+        d, dmin = _f16_at(b[..., 0:2])[..., None], _f16_at(b[..., 2:4])[..., None]
+        return ((d * sc)[..., None] * q - (dmin * mn)[..., None]).reshape(n, k)
+    b = blocks.reshape(n, k // 256, 210)
+    ql, qh = b[..., :128].reshape(n, k // 256, 2, 2, 32).to(torch.int64), b[..., 128:192].reshape(n, k // 256, 2, 32).to(torch.int64)
+    low = torch.stack([ql[..., 0, :] & 15, ql[..., 1, :] & 15, ql[..., 0, :] >> 4, ql[..., 1, :] >> 4], dim=3)
+    high = torch.stack([(qh >> s) & 3 for s in (0, 2, 4, 6)], dim=3)
+    q = ((low | (high << 4)) - 32).double().reshape(n, k // 256, 16, 16)
+    sc = b[..., 192:208].contiguous().view(torch.int8).double()
+    return (_f16_at(b[..., 208:210])[..., None, None] * sc[..., None] * q).reshape(n, k)
+
+
+def _weights(fmt, n, k, gen):
+    return _dequantize(fmt, _blocks(fmt, n, k, gen), n, k)
+
+
+def _gated(gate_up):
+    g, u = gate_up.chunk(2, dim=-1)
+    return torch.nn.functional.silu(g) * u
+
+
+def _exact_moe(c, gen):
+    e, h, f = c["experts"], c["hidden"], c["ffn"]
+    gate_up, down = _blocks("q4_k", e * 2 * f, h, gen).chunk(e), _blocks("q4_k", e * h, f, gen).chunk(e)
+    x = _rows(c["rows"], h, gen).double()
+    logits = torch.randn(c["rows"], e, generator=gen, device="cuda") + 0.3 * torch.randn(e, generator=gen, device="cuda")
+    weights, ids = torch.softmax(logits, dim=-1).topk(c["top_k"], dim=-1)
+    weights = (weights / weights.sum(dim=-1, keepdim=True)).double()
+    y = torch.zeros_like(x)
+    for i in range(e):
+        row, choice = (ids == i).nonzero(as_tuple=True)
+        if len(row):
+            out = _gated(x[row] @ _dequantize("q4_k", gate_up[i], 2 * f, h).t()) @ _dequantize("q4_k", down[i], h, f).t()
+            y.index_add_(0, row, out * weights[row, choice][:, None])
+    return y
+
+
+def _exact_step(c, gen):
+    h, d, b, hq, hkv, f = c["hidden"], HEAD_DIM, c["rows"], c["q_heads"], c["kv_heads"], c["ffn"]
+    half = torch.arange(0, d, 2, device="cuda", dtype=torch.float64) / d
+    ang = (c["n_ctx"] - 1) / (500000.0 ** half)
+    cos, sin = (torch.cat([t, t]).to(torch.bfloat16).double() for t in (ang.cos(), ang.sin()))
+    layers = []
+    for _ in range(c["layers"]):
+        layers.append([_weights("q4_k", n, k, gen) for n, k in (((hq + 2 * hkv) * d, h), (h, hq * d), (2 * f, h), (h, f))]
+                      + [(1 + 0.1 * torch.randn(h, generator=gen, device="cuda")).to(torch.bfloat16).double() for _ in range(2)]
+                      + [torch.randn(b, hkv, c["context"], d, generator=gen, device="cuda").to(torch.bfloat16).double() for _ in range(2)])
+    head = _weights("q6_k", c["vocab"], h, gen)
+    final = (1 + 0.1 * torch.randn(h, generator=gen, device="cuda")).to(torch.bfloat16).double()
+    emb = torch.randn(c["vocab"], h, generator=gen, device="cuda", dtype=torch.bfloat16)
+    x = emb[torch.randint(0, c["vocab"], (b,), generator=gen, device="cuda")].double()
+
+    def norm(v, w):
+        return v / torch.sqrt((v * v).mean(dim=-1, keepdim=True) + EPS) * w
+
+    def rope(t):
+        return t * cos + torch.cat([-t[..., d // 2:], t[..., :d // 2]], dim=-1) * sin
+
+    for qkv, o, gate_up, down, attn_norm, mlp_norm, kc, vc in layers:
+        q, k, v = (norm(x, attn_norm) @ qkv.t()).view(b, hq + 2 * hkv, d).split([hq, hkv, hkv], dim=1)
+        kc[:, :, c["n_ctx"] - 1], vc[:, :, c["n_ctx"] - 1] = rope(k), v
+        q = rope(q).view(b, hkv, hq // hkv, d)
+        p = torch.softmax(q @ kc[:, :, :c["n_ctx"]].transpose(2, 3) / math.sqrt(d), dim=-1)
+        x = x + (p @ vc[:, :, :c["n_ctx"]]).reshape(b, hq * d) @ o.t()
+        x = x + _gated(norm(x, mlp_norm) @ gate_up.t()) @ down.t()
+    return [norm(x, final) @ head.t()] + [t for L in layers for t in L[6:]]
+
+
+def exact(case, seed):
+    c, kind = dict(case), case["kind"]
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    if kind == "linear":
+        bias = torch.randn(c["n"], generator=gen, device="cuda").to(DTYPES[c["x"]]).double() if c["bias"] else 0.0
+        w = _weights(c["fmt"], c["n"], c["k"], gen)
+        return _rows(c["rows"], c["k"], gen, DTYPES[c["x"]]).double() @ w.t() + bias
+    if kind == "layer":
+        qkv, o, gate_up, down = (_weights(c["fmt"], n, k, gen) for n, k in _layer_shapes(c))
+        x, att, h = (_rows(c["rows"], c["hidden"], gen).double() for _ in range(3))
+        return [x @ qkv.t(), att @ o.t(), _gated(h @ gate_up.t()) @ down.t()]
+    if kind == "mlp":
+        gate, up, down = (_weights(c["fmt"], n, k, gen) for n, k in ((c["ffn"], c["hidden"]), (c["ffn"], c["hidden"]), (c["hidden"], c["ffn"])))
+        x = _rows(c["rows"], c["hidden"], gen).double()
+        return (torch.nn.functional.silu(x @ gate.t()) * (x @ up.t())) @ down.t()
+    if kind == "moe":
+        return _exact_moe(c, gen)
+    if kind == "step":
+        return _exact_step(c, gen)
+    ys = []
+    for _ in range(c["layers"]):
+        shapes = _layer_shapes(c)
+        ws = [_weights(c["fmt"], n, k, gen) for n, k in shapes]
+        ys += [(_rows(c["rows"], k, gen).double() @ w.t()).cpu() for w, (n, k) in zip(ws, shapes)]
+    return ys
