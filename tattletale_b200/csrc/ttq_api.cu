@@ -589,12 +589,23 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         const int64_t n = v ? atoll(v) : 0;
         return n >= 1 ? n : 5;
     }();
-    // Q8_0 / Q6_K: the integer decode kernel serves 16 rows per pass; from 9 rows the fused tensor-core GEMM is used
+    // Q8_0 / Q6_K: the integer decode kernel serves 16 rows per pass; from 9 rows the tensor-core kernels are used
     const int64_t gemm_min_m = w->fmt == TTQ_FMT_Q4_K ? GEMM_MIN_M : (GEMM_MIN_M > 9 ? GEMM_MIN_M : 9);
     if (M >= gemm_min_m && use_gemm && gemm_supported(w->fmt)) {
         // prefill / larger batches: tensor-core path
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
+        // Up to 192 rows the tensor-memory kernel (4096 -> 28672, us, it against the shared-memory GEMM: 30 / 65 at 17 rows, 51 / 69
+        // at 128, 75 / 81 at 192); up to 256 while there are fewer 128-row groups of weights than SMs, where its even split of K
+        // wins (4096 -> 6144 at 256 rows 38 / 46, 14336 -> 4096 54 / 58; 4096 -> 28672: 85 / 82).  Beyond, every block of rows would
+        // expand the weights again.
+        if (M <= 192 || (M <= 256 && w->N <= (int64_t)128 * ctx->sms)) {
+            cudaError_t e = launch_gemm_ts(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
+                                           ctx->split_counters_cap, st, &launches);
+            ctx->launches += launches;
+            if (e == cudaSuccess) return TTQ_OK;
+            if (e != cudaErrorNotSupported) return cuda_fail(ctx, e, "linear forward (tensor-memory GEMM) launch");
+        }
         cudaError_t e = launch_gemm(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->trace, st, &launches);
         ctx->launches += launches;
         if (e != cudaSuccess) return cuda_fail(ctx, e, "linear forward (GEMM) launch");

@@ -158,11 +158,23 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[16]) {
 // silu(x[k]) * x[K + k] (the gated-MLP activation, fused into the conversion).
 // `kmap` = 1 selects the Q6_K stage order: slot j of stage s = 2s' + n holds window n of the 16-wide sub-block
 // 4s' + 8 (j & 1) + (j >> 1) (low nibbles: set s', high nibbles: set s' + 2 of the packed chunk).
+// `kmap` = 2 (Q4_K), 3 (Q6_K), 4 (Q8_0): the slot order of the tensor-memory expansion of ttq_gemm_ts.cu, slot
+// p = 4 (u >> 1) + 2 hi + (u & 1) for run `hi` of group u.
+__device__ __forceinline__ int xh_slot_k(int kmap, int s, int j) {
+    const int jj = (j & 4) | ((j & 1) << 1) | ((j >> 1) & 1);  // 2 u + hi
+    if (kmap == 0) return 32 * j + 8 * s;
+    if (kmap == 2) return 32 * jj + 8 * s;
+    if (kmap == 4) return 32 * ((jj >> 1) + 4 * (jj & 1)) + 8 * s;
+    const int q = kmap == 3 ? jj : j;
+    return 16 * (4 * (s >> 1) + 8 * (q & 1) + (q >> 1)) + 8 * (s & 1);
+}
 template <bool GATED>
 __global__ void __launch_bounds__(256) xh_prep_kernel(const void *__restrict__ x, int x_dt, int64_t M, int64_t Mp, int64_t K,
                                                       int64_t Kp, int64_t ldx, __half *__restrict__ xh,
                                                       const int *__restrict__ row_src, const int *__restrict__ rows_used,
-                                                      int rows_unit, int kmap) {
+                                                      int rows_unit, int kmap, int early) {
+    // A grid that is resident as a whole lets the GEMM be set up right away; it fits beside it on an SM.
+    if (early) grid_launch_dependents();
     grid_dependency_wait();  // x, the routing tables and the image buffer belong to preceding kernels until here
     const int64_t chunks_per_row = Kp / 8;
     const int64_t total = Mp * chunks_per_row;
@@ -174,7 +186,7 @@ __global__ void __launch_bounds__(256) xh_prep_kernel(const void *__restrict__ x
         if (mi >= m_used) continue;
         const int64_t sb = it >> 2;
         const int s = (int)(it & 3);
-        const int64_t k0 = kmap == 0 ? sb * 256 + 32 * j + 8 * s : sb * 256 + 16 * (4 * (s >> 1) + 8 * (j & 1) + (j >> 1)) + 8 * (s & 1);
+        const int64_t k0 = sb * 256 + xh_slot_k(kmap, s, j);
         // source row: the image row itself, or the row the routing table names (negative = padding)
         int64_t m = mi;
         if (row_src != nullptr) {
@@ -235,7 +247,7 @@ __global__ void __launch_bounds__(256) xh_prep_kernel(const void *__restrict__ x
     }
     // only now may the GEMM be set up: its one-per-SM CTAs would otherwise take the SMs from the waves of this
     // bandwidth-bound pass that are still queued
-    grid_launch_dependents();
+    if (!early) grid_launch_dependents();
 }
 
 struct GemmParams {
@@ -1337,6 +1349,18 @@ cudaError_t launch_pair(const GemmParams &p, int sms, cudaStream_t st) {
 
 }  // namespace
 
+// fp16 images of the rows of a.x, padded with zero rows to Mp (a multiple of 8).
+cudaError_t launch_xh_images(const LinearArgs &a, int64_t Mp, int64_t Kp, __half *xh, int sms, int kmap, cudaStream_t st) {
+    const int64_t chunks = Mp * (Kp / 8);
+    // up to three passes of one CTA per SM: resident as a whole beside the GEMM that is set up meanwhile
+    const int early = chunks <= (int64_t)sms * 768 ? 1 : 0;
+    const int64_t cap = early ? sms : sms * 16;
+    const unsigned grid = (unsigned)((chunks + 255) / 256 < cap ? (chunks + 255) / 256 : cap);
+    const int *no_tab = nullptr;
+    return a.gated ? launch_pdl(xh_prep_kernel<true>, dim3(grid), dim3(256), 0, st, a.x, a.x_dt, a.M, Mp, a.K, Kp, a.ldx, xh, no_tab, no_tab, 0, kmap, early)
+                   : launch_pdl(xh_prep_kernel<false>, dim3(grid), dim3(256), 0, st, a.x, a.x_dt, a.M, Mp, a.K, Kp, a.ldx, xh, no_tab, no_tab, 0, kmap, early);
+}
+
 bool gemm_supported(int fmt) { return fmt == TTQ_FMT_Q4_K || fmt == TTQ_FMT_Q8_0 || fmt == TTQ_FMT_Q6_K; }
 
 // Rows of the fp16 weight images the plain mode reads: output features padded to whole 256-row tiles.
@@ -1376,9 +1400,9 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
         const unsigned grid = (unsigned)((chunks + 255) / 256 < sms * 16 ? (chunks + 255) / 256 : sms * 16);
         const int *no_tab = nullptr;
         cudaError_t e = a.gated ? launch_pdl(xh_prep_kernel<true>, dim3(grid), dim3(256), 0, st, (const void *)xs, a.x_dt, Ms, Mp, a.K, Kp, a.ldx,
-                                             xh, no_tab, no_tab, 0, kmap)
+                                             xh, no_tab, no_tab, 0, kmap, 0)
                                 : launch_pdl(xh_prep_kernel<false>, dim3(grid), dim3(256), 0, st, (const void *)xs, a.x_dt, Ms, Mp, a.K, Kp, a.ldx,
-                                             xh, no_tab, no_tab, 0, kmap);
+                                             xh, no_tab, no_tab, 0, kmap, 0);
         if (e != cudaSuccess) return e;
         ++*launches;
         GemmParams p;
@@ -1571,9 +1595,9 @@ cudaError_t launch_gemm_grouped(const GroupedArgs &g, __half *xh, int sms, int *
     const int64_t chunks = g.Mp * (Kp / 8);
     const unsigned grid = (unsigned)((chunks + 255) / 256 < sms * 16 ? (chunks + 255) / 256 : sms * 16);
     cudaError_t e = g.gated ? launch_pdl(xh_prep_kernel<true>, dim3(grid), dim3(256), 0, st, g.x, g.x_dt, g.x_rows, g.Mp, g.K, Kp, g.ldx, xh,
-                                         g.row_src, g.rows_total, 1, 0)
+                                         g.row_src, g.rows_total, 1, 0, 0)
                             : launch_pdl(xh_prep_kernel<false>, dim3(grid), dim3(256), 0, st, g.x, g.x_dt, g.x_rows, g.Mp, g.K, Kp, g.ldx, xh,
-                                         g.row_src, g.rows_total, 1, 0);
+                                         g.row_src, g.rows_total, 1, 0, 0);
     if (e != cudaSuccess) return e;
     ++*launches;
     GemmParams p;

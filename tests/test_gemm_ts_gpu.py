@@ -1,0 +1,53 @@
+"""The GEMM that expands packed weights into tensor memory, at the sizes where its split can go wrong, against the CPU checker.
+
+Row counts around the 16-row granularity of the activation block, the switch from two accumulator sets to one (128) and the
+largest block (256); weight rows that end inside a 16-row tile and inside a 128-row group; one super-block, an odd number,
+and enough to cut every output tile over several CTAs (partial sums and arrival counters: a second call must agree bit for
+bit).  Weights and activations are rounded to fp16 (2^-11 each, independent), sums are fp32: expected relative L2 error
+2e-4 to 4e-4, bar 1e-3."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import tattletale_b200 as ttq
+from conftest import rel_l2
+from gpu_util import ALL_FMTS, FMT_IDS, OFMT, make_weight, make_x, odt, x_bits
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-3
+
+
+@pytest.mark.parametrize("fmt", ALL_FMTS, ids=FMT_IDS)
+@pytest.mark.parametrize("n,k,m", [(16, 256, 17), (100, 512, 32), (130, 768, 33), (1000, 1024, 48), (256, 2304, 112), (4096, 512, 128),
+                                   (264, 1280, 129), (3000, 2560, 144), (128, 4096, 255), (512, 256, 256)])
+def test_matches_checker(ctx, fmt, n, k, m):
+    dtype = torch.float16 if m % 2 else torch.bfloat16
+    blocks = make_weight(fmt, n, k, seed=n + k + m)
+    x = make_x(m, k, seed=m + 1, dtype=dtype)
+    bias = torch.from_numpy(np.random.default_rng(m).normal(0, 0.1, n).astype(np.float32))
+    lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks), k, bias=bias.cuda())
+    xd = x.cuda()
+    y = lin.forward(xd, out_dtype=torch.float32)
+    again = lin.forward(xd, out_dtype=torch.float32)
+    ctx.check_device_status()
+    want = oracle.linear(OFMT[fmt], blocks, x_bits(x), odt(dtype), bias.numpy())
+    assert rel_l2(y.cpu().numpy(), want) < TOL
+    assert torch.equal(y, again)
+    lin.close()
+
+
+@pytest.mark.parametrize("fmt", ALL_FMTS, ids=FMT_IDS)
+def test_rows_of_a_wider_matrix(ctx, fmt):
+    """x and y as column slices of wider tensors: row pitches larger than the row, addresses off the 16-byte grid."""
+    n, k, m = 200, 512, 50
+    blocks = make_weight(fmt, n, k, seed=5)
+    wide = make_x(m, k + 9, seed=6).cuda()
+    x = wide[:, 3:3 + k]
+    out = torch.zeros(m, n + 5, dtype=torch.bfloat16, device="cuda")
+    lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks), k)
+    want = lin.forward(x.contiguous())
+    lin.forward(x, out=out[:, :n])
+    ctx.check_device_status()
+    assert torch.equal(out[:, :n], want) and not out[:, n:].any()
+    lin.close()
