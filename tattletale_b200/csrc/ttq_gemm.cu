@@ -114,6 +114,14 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
+// One lane of a converged warp.  tcgen05.mma and bulk copies take their operands from uniform registers: issued by an elected
+// lane of a warp that walks its loop as a whole they are one instruction each (17 cycles for N = 16, the tensor core's own
+// time from N = 64), from a branch on the lane number the compiler makes a loop of about 100 cycles of each.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -664,7 +672,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                     tw0 = global_ns();
                 }
                 const uint32_t a_stage = stages_u32 + stage * C::STAGE_BYTES;
-                if (dw == 0 && my_sub == 0 && lane == 0) {
+                if (dw == 0 && my_sub == 0 && elect_one()) {
                     // the activation tile of this stage: one bulk copy, counted on the same full barrier
                     mbar_expect_tx(full_bar + 8 * stage, b_bytes);
                     bulk_g2s(a_stage + C::A_BYTES, bsrc0 + it * b_it_stride, b_bytes, full_bar + 8 * stage);
@@ -769,17 +777,17 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
         }
     } else {
         // ------------------------------------------------------------------ MMA issue
-        if (lane == 0) {
+        {
             bool alive = true;
             const uint32_t idesc = idesc_f16(128 * NSUB);
             int git = 0, tcount = 0;
-            const bool tr = p.trace != nullptr && blockIdx.x == 0;
+            const bool tr = p.trace != nullptr && blockIdx.x == 0 && lane == 0;
             unsigned long long t_start = tr ? global_ns() : 0, t_full = 0, t_acc = 0, t_issue = 0;
             for (int64_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, tcount++) {
                 const int buf = tcount % C::NACC, use = tcount / C::NACC;
                 // the epilogue must have drained this accumulator set (its previous use)
                 unsigned long long t0 = tr ? global_ns() : 0;
-                if (use >= 1 && alive) alive = mbar_wait_bounded(acce_bar + 8 * buf, (uint32_t)((use - 1) & 1), p.status);
+                if (use >= 1 && alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded(acce_bar + 8 * buf, (uint32_t)((use - 1) & 1), p.status));
                 if (tr) t_acc += global_ns() - t0;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS);
@@ -787,29 +795,32 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (tr) t0 = global_ns();
-                    if (alive) alive = mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status);
+                    if (alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
                     if (tr) {
                         t_full += global_ns() - t0;
                         t0 = global_ns();
                     }
                     tc_fence_after();
                     const uint32_t a_stage = stages_u32 + stage * C::STAGE_BYTES;
-                    // N side: the 128 * NSUB expanded weight rows of the stage (sub-tiles are contiguous 8-row atoms)
-                    const uint64_t wdesc = smem_desc_sw128(a_stage);
+                    if (elect_one()) {
+                        // N side: the 128 * NSUB expanded weight rows of the stage (sub-tiles are contiguous 8-row atoms)
+                        const uint64_t wdesc = smem_desc_sw128(a_stage);
 #pragma unroll
-                    for (int hb = 0; hb < C::MH; hb++) {
-                        if (hb >= mh) break;
-                        // M side: 128 activation rows (a 64-row tile leaves lanes 64..127 unused)
-                        const uint64_t xdesc = smem_desc_sw128(a_stage + C::A_BYTES + hb * (128 * 128));
+                        for (int hb = 0; hb < C::MH; hb++) {
+                            if (hb >= mh) break;
+                            // M side: 128 activation rows (a 64-row tile leaves lanes 64..127 unused)
+                            const uint64_t xdesc = smem_desc_sw128(a_stage + C::A_BYTES + hb * (128 * 128));
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++)  // 16 K values = 32 bytes along the swizzled row per instruction
-                            umma_f16(tmem_d + (uint32_t)(hb * 128 * NSUB), xdesc + (uint64_t)(2 * kk), wdesc + (uint64_t)(2 * kk), idesc,
-                                     (it > 0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; kk++)  // 16 K values = 32 bytes along the swizzled row per instruction
+                                umma_f16(tmem_d + (uint32_t)(hb * 128 * NSUB), xdesc + (uint64_t)(2 * kk), wdesc + (uint64_t)(2 * kk), idesc,
+                                         (it > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        umma_commit(empty_bar + 8 * stage);
+                        if (it == iters - 1) umma_commit(accf_bar + 8 * buf);
                     }
-                    umma_commit(empty_bar + 8 * stage);
+                    __syncwarp();
                     if (tr) t_issue += global_ns() - t0;
                 }
-                umma_commit(accf_bar + 8 * buf);
             }
             if (tr) {
                 // timeline entry of kind 3: start, end, time the MMA lane waited for operands / for the epilogue, stages issued
@@ -845,6 +856,8 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
 // CTAs at the same offsets and are signalled by ONE tcgen05.commit with cluster multicast (an arrive, not a load);
 // `acc_empty[set]` lives in the first CTA and counts the epilogue warps of both.  No TMA or bulk load uses multicast.
 // Dense Q4_K only, no K split; every wait is bounded.
+// Measured at 2048 rows (us; with the MMAs issued from a branch on the lane number in brackets, where each cost the issuing lane
+// more than the tensor core): 4096 -> 28672 360 (419), 14336 -> 4096 193 (226), 4096 -> 4096 59 (70) = 1336, 1245, 1166 TFLOP/s.
 // ================================================================================================================
 constexpr int GP_STAGE_W = 128 * 128;   // 128 expanded weight rows x 64 fp16
 constexpr int GP_STAGE_X = 2 * 128 * 128;   // two blocks of 128 activation rows x 64 fp16
@@ -1129,7 +1142,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                     tw0 = global_ns();
                 }
                 const uint32_t w_stage = stages_u32 + stage * GP_STAGE;
-                if (dw == 0 && lane == 0) {
+                if (dw == 0 && elect_one()) {
                     // the first CTA's copy is counted on `full` itself, the second CTA's on its local barrier (forwarded below)
                     const uint32_t bar = (rank == 0 ? full_bar : act_bar) + 8 * stage;
                     mbar_expect_tx(bar, (uint32_t)mh * 16384u);
@@ -1189,16 +1202,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
         }
     } else if (rank == 0) {
         // ------------------------------------------------------------------ MMA issue (first CTA of the pair)
-        if (lane == 0) {
+        {
             bool alive = true;
             constexpr uint32_t idesc = idesc_f16_pair(256);
             int git = 0, tcount = 0;
-            const bool tr = p.trace != nullptr && pair == 0;
+            const bool tr = p.trace != nullptr && pair == 0 && lane == 0;
             unsigned long long t_start = tr ? global_ns() : 0, t_full = 0, t_acc = 0, t_issue = 0;
             for (int64_t tile = pair; tile < n_otiles; tile += n_pairs, tcount++) {
                 // both CTAs' epilogue warps have drained the accumulators of the previous tile
                 unsigned long long t0 = tr ? global_ns() : 0;
-                if (tcount >= 1 && alive) alive = mbar_wait_bounded_cluster(acce_bar, (uint32_t)((tcount - 1) & 1), p.status);
+                if (tcount >= 1 && alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded_cluster(acce_bar, (uint32_t)((tcount - 1) & 1), p.status));
                 if (tr) t_acc += global_ns() - t0;
                 tc_fence_after();
                 int64_t n_tile_c, m_tile_c;
@@ -1206,24 +1219,27 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (tr) t0 = global_ns();
-                    if (alive) alive = mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status);
+                    if (alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
                     if (tr) {
                         t_full += global_ns() - t0;
                         t0 = global_ns();
                     }
                     tc_fence_after();
-                    const uint32_t w_stage = stages_u32 + stage * GP_STAGE;
-                    const uint64_t wdesc = smem_desc_sw128(w_stage);
-                    for (int hb = 0; hb < mh; hb++) {
-                        const uint64_t xdesc = smem_desc_sw128(w_stage + GP_STAGE_W + hb * 16384);
+                    if (elect_one()) {
+                        const uint32_t w_stage = stages_u32 + stage * GP_STAGE;
+                        const uint64_t wdesc = smem_desc_sw128(w_stage);
+                        for (int hb = 0; hb < mh; hb++) {
+                            const uint64_t xdesc = smem_desc_sw128(w_stage + GP_STAGE_W + hb * 16384);
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++)
-                            umma_f16_pair(tmem_base + (uint32_t)(hb * 256), xdesc + (uint64_t)(2 * kk), wdesc + (uint64_t)(2 * kk), idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; kk++)
+                                umma_f16_pair(tmem_base + (uint32_t)(hb * 256), xdesc + (uint64_t)(2 * kk), wdesc + (uint64_t)(2 * kk), idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        umma_commit_pair(empty_bar + 8 * stage);
+                        if (it == iters - 1) umma_commit_pair(accf_bar);
                     }
-                    umma_commit_pair(empty_bar + 8 * stage);
+                    __syncwarp();
                     if (tr) t_issue += global_ns() - t0;
                 }
-                umma_commit_pair(accf_bar);
             }
             if (tr) {
                 // timeline entry of kind 3, as in the one-CTA kernel
@@ -1347,6 +1363,16 @@ cudaError_t launch_pair(const GemmParams &p, int sms, cudaStream_t st) {
     return cudaLaunchKernelEx(&cfg, gemm_q4k_pair_kernel, p);
 }
 
+// Time of the pair kernel over `cols` weight-tile columns, in pipeline stages of the one-CTA kernel: the load of the first
+// pair, tiles dealt round-robin, full tiles (512 rows) before half tiles (256 rows).
+double pair_makespan(int64_t cols, int64_t m_full, int64_t m_half, int64_t slots, double iters) {
+    const double c_full = 0.73 * iters + 8.0, c_half = 0.52 * iters + 6.0;
+    const int64_t nf = cols * m_full, nt = nf + cols * m_half;
+    double t = 0;
+    for (int64_t k = 0; slots > 0 && k < nt; k += slots) t += k < nf ? c_full : c_half;
+    return t;
+}
+
 }  // namespace
 
 // fp16 images of the rows of a.x, padded with zero rows to Mp (a multiple of 8).
@@ -1383,11 +1409,24 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
     // a CTA with two sub-tiles does twice the work per activation stage in about 1.65x the time of one (measured: five
     // rounds of one sub-tile against three of two on 4096 -> 28672 at 768 rows take 221 against 203 us; the single
     // sub-tile is expanded by two warp groups on alternating stages)
+    // TTQ_GEMM_PAIR: 0 never, 1 (default) where the model prefers it, 2 wherever it applies
+    static const int pair_mode = []() {
+        const char *v = getenv("TTQ_GEMM_PAIR");
+        return v ? atoi(v) : 1;
+    }();
     const int64_t mt = (a.M + BM - 1) / BM;
     const int64_t tiles1 = ((a.N + 127) / 128) * mt, tiles2 = ((a.N + 255) / 256) * mt;
     const double cost1 = (double)((tiles1 + sms - 1) / sms), cost2 = 1.65 * (double)((tiles2 + sms - 1) / sms);
     int nsub = (a.N > 128 && cost2 < cost1) ? 2 : 1;
     if (force_nsub == 1 || force_nsub == 2) nsub = force_nsub;
+    // (the pair kernel's tiles are two sub-tiles wide: where a single sub-tile would only spare the one-CTA kernel a ragged round,
+    // the pair may still be the cheaper one -- 4096 -> 6144 at 2048 rows: 110 against 136 us)
+    if (nsub == 1 && pair_mode > 0 && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && a.N > 128 && force_nsub == 0) {
+        const double iters = (double)a.SBp * 4;
+        const int64_t slots = pair_slots(sms), mp = mt * 256;
+        if (slots > 0 && tiles2 > sms / 2 && pair_makespan((a.N + 255) / 256, mp / 512, mp % 512 ? 1 : 0, slots, iters) < cost1 * (iters + 8.0) / 1.65)
+            nsub = 2;
+    }
     if (plain || fmt != TTQ_FMT_Q4_K) nsub = 2;  // plain: no conversion work to balance; Q8_0 / Q6_K: one variant
     int64_t slab = (xh_capacity / Kp) / BM * BM;  // rows per pass
     if (slab < BM) return cudaErrorInvalidValue;
@@ -1511,25 +1550,14 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
             }
         }
         // The two-CTA kernel (dense Q4_K, more than 128 rows, no K split): a pair's tile is 256 weight rows x 512
-        // activation rows, and a stage of it takes about 0.85 of the one-CTA kernel's stage for twice the work (measured
-        // at 4096 -> 28672, 2048 rows); a half tile (256 rows) about 0.6.  With 74 slots the rounds are coarser, so the
+        // activation rows, and a stage of it takes about 0.73 of the one-CTA kernel's stage for twice the work (measured
+        // at 4096 -> 28672, 2048 rows); a half tile (256 rows) about 0.52.  With 74 slots the rounds are coarser, so the
         // model prices both kernels, each with its best tail, and takes the cheaper.  The pair's load is that of the
         // first pair: tiles are dealt round-robin, full tiles first.
-        // TTQ_GEMM_PAIR: 0 never, 1 (default) where the model prefers it, 2 wherever it applies
-        static const int pair_mode = []() {
-            const char *v = getenv("TTQ_GEMM_PAIR");
-            return v ? atoi(v) : 1;
-        }();
         bool use_pair = false;
         if (pair_mode > 0 && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && nsub == 2 && splits == 1) {
             const int64_t slots = pair_slots(sms), m_full = Mp / 512, m_half = (Mp % 512) ? 1 : 0;
-            const double c_full = 0.85 * iters + 8.0, c_half = 0.6 * iters + 6.0;
-            auto makespan = [&](int64_t cols) {
-                const int64_t nf = cols * m_full, nt = nf + cols * m_half;
-                double t = 0;
-                for (int64_t k = 0; slots > 0 && k < nt; k += slots) t += k < nf ? c_full : c_half;
-                return t;
-            };
+            auto makespan = [&](int64_t cols) { return pair_makespan(cols, m_full, m_half, slots, iters); };
             double best = makespan(n_tiles);
             int64_t best_cols = 0;
             int best_runs = 1;
