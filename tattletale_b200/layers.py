@@ -23,7 +23,18 @@ def _dt(t: torch.dtype) -> int:
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the current stream's handle without the Stream object around it (about 2 us a call)
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+def _rows_of(x: torch.Tensor, k: int) -> tuple[torch.Tensor, int]:
+    """``x`` as rows of ``k`` consecutive values, and their pitch (``k`` for a single row)."""
+    x2 = x if x.dim() == 2 else x.reshape(-1, k)
+    pitch, unit = x2.stride()
+    if unit != 1:
+        return x2.contiguous(), k
+    return x2, pitch if x2.shape[0] > 1 else k
 
 
 class Context:
@@ -177,24 +188,27 @@ class QuantLinear:
                 out: Optional[torch.Tensor] = None, use_bias: bool = True) -> torch.Tensor:
         if not x.is_cuda:
             raise TtqError(1, "x must live on the context's CUDA device (use forward_host for host buffers)")
-        if x.shape[-1] != self.in_features:
-            raise TtqError(2, f"x has {x.shape[-1]} input features, the layer has {self.in_features}")
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        m = x2.shape[0]
-        odt = out_dtype or x.dtype
+        shape, k, n = x.shape, self.in_features, self.out_features
+        if shape[-1] != k:
+            raise TtqError(2, f"x has {shape[-1]} input features, the layer has {k}")
+        flat = len(shape) == 2
+        x2, ldx = _rows_of(x, k)
+        m, device = x2.shape[0], x.device
         if out is None:
-            out = torch.empty((m, self.out_features), dtype=odt, device=x.device)
-        y2 = out.reshape(-1, self.out_features)
+            y2 = torch.empty((m, n), dtype=out_dtype or x.dtype, device=device)
+            out, ldy = (y2 if flat else y2.reshape(*shape[:-1], n)), n
+        else:
+            y2 = out.reshape(-1, n)
+            out, ldy = out.reshape(*shape[:-1], n), y2.stride(0) if m > 1 else n
         b = self.bias if use_bias else None
-        st = self.ctx._lib.ttq_linear_forward(
-            self.ctx.handle, self.handle, x2.data_ptr(), _dt(x2.dtype), m, x2.stride(0) if m > 1 else self.in_features,
+        ctx = self.ctx
+        st = ctx._lib.ttq_linear_forward(
+            ctx.handle, self.handle, x2.data_ptr(), _dt(x2.dtype), m, ldx,
             None if b is None else b.data_ptr(), _lib.DT_F32 if b is None else _dt(b.dtype),
-            y2.data_ptr(), _dt(y2.dtype), y2.stride(0) if m > 1 else self.out_features, _stream_ptr(x.device))
-        check(self.ctx.handle, st)
-        return out.reshape(*lead, self.out_features)
+            y2.data_ptr(), _dt(y2.dtype), ldy, _stream_ptr(device))
+        if st != 0:
+            check(ctx.handle, st)
+        return out
 
     __call__ = forward
 
@@ -218,20 +232,23 @@ class QuantLinear:
         of the gated MLP (mlp.nim:56-60) folded into the input conversion of this (down) projection."""
         if gate_up.shape[-1] != 2 * self.in_features:
             raise TtqError(2, f"gate_up has {gate_up.shape[-1]} columns, expected {2 * self.in_features}")
-        x2 = gate_up.reshape(-1, 2 * self.in_features)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        m = x2.shape[0]
+        shape, n = gate_up.shape, self.out_features
+        x2, ldx = _rows_of(gate_up, 2 * self.in_features)
+        m, device = x2.shape[0], gate_up.device
         if out is None:
-            out = torch.empty((m, self.out_features), dtype=out_dtype or gate_up.dtype, device=gate_up.device)
-        y2 = out.reshape(-1, self.out_features)
-        b = self.bias
-        st = self.ctx._lib.ttq_linear_forward_gated(
-            self.ctx.handle, self.handle, x2.data_ptr(), _dt(x2.dtype), m, x2.stride(0) if m > 1 else 2 * self.in_features,
+            y2 = torch.empty((m, n), dtype=out_dtype or gate_up.dtype, device=device)
+            out, ldy = (y2 if len(shape) == 2 else y2.reshape(*shape[:-1], n)), n
+        else:
+            y2 = out.reshape(-1, n)
+            out, ldy = out.reshape(*shape[:-1], n), y2.stride(0) if m > 1 else n
+        b, ctx = self.bias, self.ctx
+        st = ctx._lib.ttq_linear_forward_gated(
+            ctx.handle, self.handle, x2.data_ptr(), _dt(x2.dtype), m, ldx,
             None if b is None else b.data_ptr(), _lib.DT_F32 if b is None else _dt(b.dtype),
-            y2.data_ptr(), _dt(y2.dtype), y2.stride(0) if m > 1 else self.out_features, _stream_ptr(gate_up.device))
-        check(self.ctx.handle, st)
-        return out.reshape(*gate_up.shape[:-1], self.out_features)
+            y2.data_ptr(), _dt(y2.dtype), ldy, _stream_ptr(device))
+        if st != 0:
+            check(ctx.handle, st)
+        return out
 
     def forward_allreduce(self, x: torch.Tensor, comm, out_dtype: Optional[torch.dtype] = None,
                           out: Optional[torch.Tensor] = None) -> torch.Tensor:
