@@ -168,93 +168,114 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[16]) {
 // 4s' + 8 (j & 1) + (j >> 1) (low nibbles: set s', high nibbles: set s' + 2 of the packed chunk).
 // `kmap` = 2 (Q4_K), 3 (Q6_K), 4 (Q8_0): the slot order of the tensor-memory expansion of ttq_gemm_ts.cu, slot
 // p = 4 (u >> 1) + 2 hi + (u & 1) for run `hi` of group u.
-__device__ __forceinline__ int xh_slot_k(int kmap, int s, int j) {
-    const int jj = (j & 4) | ((j & 1) << 1) | ((j >> 1) & 1);  // 2 u + hi
-    if (kmap == 0) return 32 * j + 8 * s;
-    if (kmap == 2) return 32 * jj + 8 * s;
-    if (kmap == 4) return 32 * ((jj >> 1) + 4 * (jj & 1)) + 8 * s;
-    const int q = kmap == 3 ? jj : j;
-    return 16 * (4 * (s >> 1) + 8 * (q & 1) + (q >> 1)) + 8 * (s & 1);
+//
+// A warp converts one super-block of one row: 512 contiguous bytes in, four runs of 128 bytes out (its four stages); the
+// eight warps of a CTA take the eight rows of a swizzle atom.  Memory-bound: 2048 rows of 28672 bf16 values, gated, move 176 MB.
+// (A thread per 16-byte slot in the order of the image took 130 us longer for those: half of every sector read, 64-bit
+// divisions per slot, 2-byte loads of gated bf16 rows.  Projections of an 8B layer at 2048 rows: 989 -> 855 us.)
+// `early`: the whole grid is resident and fits beside the GEMM that follows, which may be set up right away.
+
+// K values 8 L .. 8 L + 7 of a super-block -> stage s (window) and 16-byte slot
+__device__ __forceinline__ void xh_place(int kmap, int L, int &s, int &slot) {
+    s = L & 3;
+    int q = L >> 2;  // kmap 0, 2: sub-block = slot, resp. 2 u + hi
+    if (kmap == 4) q = 2 * (q & 3) + (q >> 2);
+    if (kmap == 1 || kmap == 3) {
+        const int b = L >> 1;  // 16-wide sub-block 4 s' + 8 hi + u
+        s = 2 * ((b >> 2) & 1) + (L & 1);
+        q = 2 * (b & 3) + (b >> 3);
+    }
+    slot = kmap >= 2 ? ((q & 4) | ((q & 1) << 1) | ((q >> 1) & 1)) : q;
+}
+__device__ __forceinline__ void xh_unpack(const uint4 &raw, int dt, float (&v)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if (dt == TTQ_DT_BF16) {
+            v[2 * q] = __uint_as_float(w[q] << 16);
+            v[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
+            v[2 * q] = f.x;
+            v[2 * q + 1] = f.y;
+        }
+    }
 }
 template <bool GATED>
 __global__ void __launch_bounds__(256) xh_prep_kernel(const void *__restrict__ x, int x_dt, int64_t M, int64_t Mp, int64_t K,
                                                       int64_t Kp, int64_t ldx, __half *__restrict__ xh,
                                                       const int *__restrict__ row_src, const int *__restrict__ rows_used,
                                                       int rows_unit, int kmap, int early) {
-    // A grid that is resident as a whole lets the GEMM be set up right away; it fits beside it on an SM.
     if (early) grid_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t SBp = (uint32_t)(Kp >> 8);
+    int s, slot;
+    xh_place(kmap, lane, s, slot);
+    const bool aligned = x_dt != TTQ_DT_F32 && ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2) | (uintptr_t)(GATED ? K * 2 : 0)) & 15) == 0;
     grid_dependency_wait();  // x, the routing tables and the image buffer belong to preceding kernels until here
-    const int64_t chunks_per_row = Kp / 8;
-    const int64_t total = Mp * chunks_per_row;
     const int64_t m_used = rows_used != nullptr ? (int64_t)(*rows_used) * rows_unit : Mp;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (int64_t)gridDim.x * blockDim.x) {
-        // consecutive threads: consecutive j, then rows, then stages (coalesced 16-byte stores per atom)
-        const int j = (int)(c & 7);
-        const int64_t mi = (c >> 3) % Mp, it = (c >> 3) / Mp;
-        if (mi >= m_used) continue;
-        const int64_t sb = it >> 2;
-        const int s = (int)(it & 3);
-        const int64_t k0 = sb * 256 + xh_slot_k(kmap, s, j);
-        // source row: the image row itself, or the row the routing table names (negative = padding)
-        int64_t m = mi;
-        if (row_src != nullptr) {
-            const int r = row_src[mi];
-            m = r < 0 ? M : (int64_t)r;
+    const uint32_t atoms = (uint32_t)((m_used < Mp ? m_used + 7 : Mp) >> 3), units = atoms * SBp;
+    // two units in flight: their loads are issued before either is converted (gated: one, two would take the registers that
+    // let this kernel sit beside the GEMM)
+    constexpr int UN = GATED ? 1 : 2;
+    for (uint32_t u0 = blockIdx.x; u0 < units; u0 += UN * gridDim.x) {
+        uint4 ga[UN], ua[UN];
+        int64_t row_m[UN];  // source row: the image row itself, or the row the routing table names; M = a row of zeros, -1 = no unit
+#pragma unroll
+        for (int i = 0; i < UN; i++) {
+            const uint32_t u = u0 + i * gridDim.x, atom = u / SBp, sb = u - atom * SBp;
+            const int64_t mi = (int64_t)atom * 8 + warp, k0 = (int64_t)sb * 256 + 8 * lane;
+            row_m[i] = -1;
+            if (u >= units || mi >= m_used || mi >= Mp) continue;
+            int64_t m = mi;
+            if (row_src != nullptr) {
+                const int r = row_src[mi];
+                m = r < 0 ? M : (int64_t)r;
+            }
+            row_m[i] = m;
+            if (m < M && aligned && k0 + 8 <= K) {
+                const uint16_t *row = reinterpret_cast<const uint16_t *>(x) + m * ldx + k0;
+                ga[i] = *reinterpret_cast<const uint4 *>(row);
+                if (GATED) ua[i] = *reinterpret_cast<const uint4 *>(row + K);
+            }
         }
-        // the 8 source values are contiguous in K: one 16-byte load when the row is aligned
-        __half src[8];
-        const bool vec = x_dt != TTQ_DT_F32 && m < M && k0 + 8 <= K &&
-                         ((reinterpret_cast<uintptr_t>(x) + (size_t)(m * ldx + k0) * 2) & 15) == 0 && (!GATED || ((K * 2) & 15) == 0);
-        if (GATED) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) src[i] = __float2half_rn(0.f);
-            if (vec && x_dt == TTQ_DT_F16) {
-                const __half *row = reinterpret_cast<const __half *>(x) + m * ldx + k0;
-                const uint4 ga = *reinterpret_cast<const uint4 *>(row), ua = *reinterpret_cast<const uint4 *>(row + K);
-                const __half2 *g2 = reinterpret_cast<const __half2 *>(&ga), *u2 = reinterpret_cast<const __half2 *>(&ua);
+        for (int i = 0; i < UN; i++) {
+            const uint32_t u = u0 + i * gridDim.x, atom = u / SBp, sb = u - atom * SBp;
+            const int64_t m = row_m[i], k0 = (int64_t)sb * 256 + 8 * lane;
+            if (m < 0) continue;
+            float v[8];
+            if (m < M && aligned && k0 + 8 <= K) {
+                xh_unpack(ga[i], x_dt, v);
+                if (GATED) {
+                    float w[8];
+                    xh_unpack(ua[i], x_dt, w);
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float2 gv = __half22float2(g2[q]), uv = __half22float2(u2[q]);
-                    src[2 * q] = __float2half_rn(gv.x / (1.f + expf(-gv.x)) * uv.x);
-                    src[2 * q + 1] = __float2half_rn(gv.y / (1.f + expf(-gv.y)) * uv.y);
+                    for (int q = 0; q < 8; q++) v[q] = v[q] / (1.f + expf(-v[q])) * w[q];
                 }
-            } else if (m < M) {
+            } else {
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (k0 + i < K) {
-                        const float gv = load_as_float(x, x_dt, m * ldx + k0 + i), uv = load_as_float(x, x_dt, m * ldx + K + k0 + i);
-                        src[i] = __float2half_rn(gv / (1.f + expf(-gv)) * uv);
+                for (int q = 0; q < 8; q++) {
+                    v[q] = 0.f;
+                    if (m < M && k0 + q < K) {
+                        v[q] = load_as_float(x, x_dt, m * ldx + k0 + q);
+                        if (GATED) v[q] = v[q] / (1.f + expf(-v[q])) * load_as_float(x, x_dt, m * ldx + K + k0 + q);
                     }
                 }
             }
-        } else if (vec) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(x) + m * ldx + k0);
-            if (x_dt == TTQ_DT_F16) {
-                *reinterpret_cast<uint4 *>(src) = raw;
-            } else {
-                const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+            // the middle two of each four change places
+            uint32_t o[4];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    src[2 * q] = __float2half_rn(__uint_as_float(w[q] << 16));
-                    src[2 * q + 1] = __float2half_rn(__uint_as_float(w[q] & 0xffff0000u));
-                }
+            for (int q = 0; q < 4; q++) {
+                const __half2 h = __floats2half2_rn(v[(q >> 1) * 4 + (q & 1)], v[(q >> 1) * 4 + (q & 1) + 2]);
+                o[q] = *reinterpret_cast<const uint32_t *>(&h);
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                float v = 0.f;
-                if (m < M && k0 + i < K) v = load_as_float(x, x_dt, m * ldx + k0 + i);
-                src[i] = __float2half_rn(v);
-            }
+            const int64_t it = (int64_t)sb * 4 + s;
+            const int64_t dst = ((it * (Mp >> 3) + atom) << 10) + (warp << 7) + ((slot ^ warp) << 4);
+            *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xh) + dst) = make_uint4(o[0], o[1], o[2], o[3]);
         }
-        __half out[8];
-#pragma unroll
-        for (int p = 0; p < 8; p++) out[p] = src[(p & 4) + ((p & 1) << 1) + ((p & 2) >> 1)];  // swap the middle two of each four
-        const int64_t dst = ((it * (Mp >> 3) + (mi >> 3)) << 10) + ((mi & 7) << 7) + ((int64_t)(j ^ (int)(mi & 7)) << 4);
-        *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xh) + dst) = *reinterpret_cast<const uint4 *>(out);
     }
-    // only now may the GEMM be set up: its one-per-SM CTAs would otherwise take the SMs from the waves of this
-    // bandwidth-bound pass that are still queued
+    // (else only now: the GEMM's one-per-SM CTAs would take the SMs from the waves of this pass that are still queued)
     if (!early) grid_launch_dependents();
 }
 
@@ -1277,17 +1298,40 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
 }
 
 // Sum of the split-K partials (+ bias) into y.
+// A CTA takes 1024 columns of one row at a time, a thread four neighbours (16-byte loads of every partial where N is a multiple
+// of four; the partials are read once, from L2 as long as they fit).
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ ws, int splits, int64_t M, int64_t Mp, int64_t N,
                                                             const void *bias, int bias_dt, void *y, int y_dt, int64_t ldy) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const int64_t total = M * N;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t m = e / N, n = e % N;
-        float acc = 0.f;
-        for (int s = 0; s < splits; s++) acc += ws[((size_t)s * Mp + m) * N + n];
-        if (bias != nullptr) acc += load_as_float(bias, bias_dt, n);
-        store_from_float(y, y_dt, m * ldy + n, acc);
+    const uint32_t pieces = (uint32_t)((N + 1023) / 1024);
+    const uint32_t total = (uint32_t)M * pieces;
+    const bool vec = (N & 3) == 0;
+    for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
+        const uint32_t m = b / pieces;
+        const int64_t n = (int64_t)(b - m * pieces) * 1024 + 4 * threadIdx.x;
+        if (n >= N) continue;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        if (vec) {
+            for (int s = 0; s < splits; s++) {
+                const float4 q = __ldcg(reinterpret_cast<const float4 *>(ws + ((size_t)s * Mp + m) * N + n));
+                acc[0] += q.x;
+                acc[1] += q.y;
+                acc[2] += q.z;
+                acc[3] += q.w;
+            }
+        } else {
+            for (int s = 0; s < splits; s++)
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (n + i < N) acc[i] += __ldcg(ws + ((size_t)s * Mp + m) * N + n + i);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (n + i >= N) continue;
+            if (bias != nullptr) acc[i] += load_as_float(bias, bias_dt, n + i);
+            store_from_float(y, y_dt, (int64_t)m * ldy + n + i, acc[i]);
+        }
     }
 }
 
@@ -1501,8 +1545,8 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
             return launch_cfg<256, 1>(q, sms, st);
         };
         auto reduce = [&](const GemmParams &q) -> cudaError_t {
-            const int64_t total = Ms * q.N;
-            const unsigned rg = (unsigned)((total + 255) / 256 < sms * 8 ? (total + 255) / 256 : sms * 8);
+            const int64_t total = Ms * ((q.N + 1023) / 1024);
+            const unsigned rg = (unsigned)(total < sms * 8 ? total : sms * 8);
             return launch_pdl(splitk_reduce_kernel, dim3(rg), dim3(256), 0, st, (const float *)q.ws, q.splits, Ms, Mp, q.N, q.bias, q.bias_dt,
                               (void *)q.y, q.y_dt, q.ldy);
         };
