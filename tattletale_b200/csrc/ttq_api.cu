@@ -1308,11 +1308,25 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
     // expert's weight rows for up to 384 of its rows); measured 5 % slower than 256-row tiles at 256 rows per
     // expert because it runs with one 128-row weight sub-tile per CTA
     int BM = mean <= 64 ? 64 : (mean <= 128 ? 128 : 256);
+    // Up to 128 rows per expert on average the tensor-memory kernel, whose even split over the SMs and 16-row tiles suit few rows
+    // per expert; above, 256-row tiles of the shared-memory GEMM expand a weight once for more rows.
+    // Measured, whole layer, us (shared-memory GEMM in brackets): 128 experts of 2048 x 768, top 8: 24 tokens 140 (249), 200 194
+    // (339), 700 261 (402), 1500 422 (485); 8 experts of 4096 x 1536, top 2: 64 tokens 75 (138), 500 125 (166).
+    bool ts = mean <= 128;
+    if (ts) BM = mean <= 8 ? 16 : (mean <= 16 ? 32 : (mean <= 48 ? 64 : 128));
     static const int force_bm = []() {
         const char *v = getenv("TTQ_MOE_BM");
         return v ? atoi(v) : 0;
     }();
-    if (force_bm == 64 || force_bm == 128 || force_bm == 256 || force_bm == 384) BM = force_bm;
+    if (force_bm == 64 || force_bm == 128 || force_bm == 256 || force_bm == 384) {
+        BM = force_bm;
+        ts = false;
+    }
+    if (ts) {
+        const int64_t groups = (2 * m->I > m->H ? 2 * m->I : m->H) / 128 + 1;
+        ts = groups * (pairs / BM + m->E + 1) <= ctx->split_counters_cap;
+        if (!ts) BM = mean <= 64 ? 64 : 128;
+    }
     const int64_t unit = BM == 384 ? 128 : BM;
     int64_t Mp = ((pairs + (int64_t)m->E * unit + unit - 1) / unit) * unit;
     if (Mp > m->rows_cap) Mp = m->rows_cap / unit * unit;
@@ -1330,6 +1344,12 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
     g.mt_group = m->route.mt_group; g.n_mt = m->route.n_mt;
     g.mt_row0 = m->route.mt_row0; g.mt_mh = m->route.mt_mh; g.rows_total = m->route.n_mt + 1; g.mt_cap = mt_cap;
     g.y = m->h1; g.y_dt = TTQ_DT_F16; g.ldy = 2 * m->I;
+    if (ts) {
+        g.ts_ws = reinterpret_cast<float *>(ctx->xh);  // (the context's image scratch: 2 x SMs x 128 rows x 128 floats are 19 of its 64 MB)
+        g.ts_ws_bytes = (size_t)ctx->xh_capacity * sizeof(__half);
+        g.ts_counters = ctx->split_counters;
+        g.ts_counters_cap = ctx->split_counters_cap;
+    }
     e = launch_gemm_grouped(g, m->xh1, ctx->sms, ctx->dev_status, st, &n);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "grouped gate|up launch");
     ctx->launches += n;

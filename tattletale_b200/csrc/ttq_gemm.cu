@@ -1662,16 +1662,23 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
 cudaError_t launch_gemm_grouped(const GroupedArgs &g, __half *xh, int sms, int *status, cudaStream_t st, int *launches) {
     *launches = 0;
     const int64_t Kp = g.SBp * TILE_K;
-    if (g.BM != 64 && g.BM != 128 && g.BM != 256 && g.BM != 384) return cudaErrorInvalidValue;
+    const bool ts = g.ts_ws != nullptr;
+    if (!ts && g.BM != 64 && g.BM != 128 && g.BM != 256 && g.BM != 384) return cudaErrorInvalidValue;
+    const int kmap = ts ? 2 : 0;
     if (g.Mp % 128 && g.Mp % g.BM) return cudaErrorInvalidValue;
     const int64_t chunks = g.Mp * (Kp / 8);
     const unsigned grid = (unsigned)((chunks + 255) / 256 < sms * 16 ? (chunks + 255) / 256 : sms * 16);
     cudaError_t e = g.gated ? launch_pdl(xh_prep_kernel<true>, dim3(grid), dim3(256), 0, st, g.x, g.x_dt, g.x_rows, g.Mp, g.K, Kp, g.ldx, xh,
-                                         g.row_src, g.rows_total, 1, 0, 0)
+                                         g.row_src, g.rows_total, 1, kmap, 0)
                             : launch_pdl(xh_prep_kernel<false>, dim3(grid), dim3(256), 0, st, g.x, g.x_dt, g.x_rows, g.Mp, g.K, Kp, g.ldx, xh,
-                                         g.row_src, g.rows_total, 1, 0, 0);
+                                         g.row_src, g.rows_total, 1, kmap, 0);
     if (e != cudaSuccess) return e;
     ++*launches;
+    if (ts) {
+        e = launch_gemm_ts_grouped(g, xh, sms, status, st);
+        if (e == cudaSuccess) ++*launches;
+        return e;
+    }
     GemmParams p;
     p.tiles = nullptr;
     p.wimg = nullptr; p.Np = 0;

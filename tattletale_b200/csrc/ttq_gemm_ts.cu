@@ -57,7 +57,12 @@ struct TsParams {
     int *status;
     int ring, bslots;  // stages of the packed rings, activation slots
     int spb;           // 64-wide slices per activation slot: 4 (a whole item), 2 or 1
-    int64_t T;  // items
+    int64_t T;  // items (grouped: per row tile)
+    // grouped (mixture-of-experts) mode, group_tiles != nullptr: a block of activation rows is a row tile of the routed row
+    // space and belongs to one of many weight matrices of one shape; tables and the number of row tiles are on the device
+    const uint8_t *const *group_tiles;
+    const int *mt_group, *mt_row0, *n_mt;
+    int64_t mt_cap;
 };
 
 __device__ __forceinline__ void ts_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -283,29 +288,31 @@ __device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane
     }
 }
 
-// position of an item inside the matrix: group of 128 weight rows, activation block, super-block
+// Position of an item: tile = outer * ni + inner, super-block.  Dense: outer = 128 weight rows, inner = activation block (the
+// blocks of one run of weights are neighbours); grouped: outer = row tile, inner = 128 weight rows of its expert.
 struct TsCursor {
-    int64_t group;
-    int mb, sb;
-    __device__ __forceinline__ void init(int64_t item, int SBp, int mbs) {
+    int64_t outer;
+    int inner, sb;
+    __device__ __forceinline__ void init(int64_t item, int SBp, int ni) {
         const int64_t tile = item / SBp;
         sb = (int)(item - tile * SBp);
-        group = tile / mbs;
-        mb = (int)(tile - group * mbs);
+        outer = tile / ni;
+        inner = (int)(tile - outer * ni);
     }
-    __device__ __forceinline__ void advance(int by, int SBp, int mbs) {
+    __device__ __forceinline__ void advance(int by, int SBp, int ni) {
         sb += by;
         while (sb >= SBp) {
             sb -= SBp;
-            if (++mb == mbs) {
-                mb = 0;
-                group++;
+            if (++inner == ni) {
+                inner = 0;
+                outer++;
             }
         }
     }
 };
 
-template <int FMT>
+// (GROUPED is a template parameter: the tables cost the registers that let the activation pass sit beside the dense form)
+template <int FMT, bool GROUPED>
 __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p) {
     constexpr int TB = tile_bytes(FMT);
     extern __shared__ uint8_t smem_raw[];
@@ -324,7 +331,23 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     volatile int64_t *last_tile = reinterpret_cast<volatile int64_t *>(base_ptr + (d_empty + 32 - base));  // [2]
     // tensor memory: `na` stages of expanded weights, `nd` accumulator sets behind them
     const int na = nb <= 64 ? 3 : 2, nd = nb <= 128 ? 2 : 1, d_col = na * TS_A_COLS;
-    const int64_t T = p.T, G = gridDim.x;
+    constexpr bool grouped = GROUPED;
+    int64_t T = p.T;
+    if (grouped) {
+        grid_dependency_wait();  // the tables are written by preceding kernels
+        const int64_t used = *p.n_mt;
+        T *= used < p.mt_cap ? used : p.mt_cap;
+    }
+    int64_t G = gridDim.x;
+    if (grouped) {
+        if (T < G) G = T;
+        if ((int64_t)blockIdx.x >= G) return;  // fewer items than CTAs: the last ones have none
+    }
+    const int ni = grouped ? (int)((p.N + TS_ROWS - 1) / TS_ROWS) : mbs;
+    auto group_of = [&](const TsCursor &c) -> int64_t { return grouped ? (int64_t)c.inner : c.outer; };
+    // first image row of a block, and how many of its rows exist
+    auto row0_of = [&](const TsCursor &c) -> int { return grouped ? p.mt_row0[c.outer] : c.inner * nb; };
+    auto rows_of = [&](const TsCursor &c) -> int { return grouped || p.M - c.inner * nb >= nb ? nb : p.M - c.inner * nb; };
     const int64_t i0 = (int64_t)blockIdx.x * T / G;
     const int n_items = (int)(((int64_t)blockIdx.x + 1) * T / G - i0);
     const int64_t first_tile = i0 / SBp;
@@ -356,8 +379,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     const uint8_t *src_ptr = nullptr;  // the next tile (nullptr: rows beyond the matrix)
     int issued = 0, i_stage = 0;
     auto locate = [&]() {
-        const int64_t rt = src.group * TS_GROUP_TILES + tau;
-        src_ptr = rt < p.NT ? p.tiles + (rt * SBp + src.sb) * (int64_t)TB : nullptr;
+        const int64_t rt = group_of(src) * TS_GROUP_TILES + tau;
+        src_ptr = nullptr;
+        if (rt < p.NT && (!grouped || src.outer * ni * SBp < T)) src_ptr = (grouped ? p.group_tiles[p.mt_group[src.outer]] : p.tiles) + (rt * SBp + src.sb) * (int64_t)TB;
     };
     auto issue_next = [&]() {
         const uint32_t bar = my_bar + 8 * i_stage;
@@ -375,7 +399,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             src.sb += 2;
             if (src_ptr != nullptr) src_ptr += 2 * TB;
         } else {
-            src.advance(2, SBp, mbs);
+            src.advance(2, SBp, ni);
             locate();
         }
     };
@@ -387,8 +411,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             fence_async_shared();
         }
         __syncwarp();
-        src.init(i0, SBp, mbs);
-        src.advance(set, SBp, mbs);
+        src.init(i0, SBp, ni);
+        src.advance(set, SBp, ni);
         locate();
         for (int s = 0; s < ring && s < my_count; s++) issue_next();
     }
@@ -408,20 +432,20 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         grid_dependency_wait();  // outputs, workspace and counters may still be in use by the preceding kernel
         bool alive = true;
         TsCursor c;
-        c.init(i0, SBp, mbs);
+        c.init(i0, SBp, ni);
         int left = n_items, seg = 0;
         const int r = warp * 32 + lane;
         while (left > 0) {
             const int run = SBp - c.sb < left ? SBp - c.sb : left;  // items of this CTA inside the tile
             const bool whole = run == SBp;
             const int buf = seg % nd, use = seg / nd;
-            const int64_t tile = c.group * mbs + c.mb;
-            const int rows = p.M - c.mb * nb < nb ? p.M - c.mb * nb : nb;
+            const int64_t tile = c.outer * ni + c.inner;
+            const int rows = rows_of(c), row0 = row0_of(c);
             unsigned others = 0;  // CTAs besides this one that hold a piece of the tile
             if (!whole && threadIdx.x == 0) others = (unsigned)(((tile + 1) * SBp * G - 1) / T - ((tile * SBp + 1) * G - 1) / T);
             if (alive) alive = ts_wait_warp(d_full + 8 * buf, (uint32_t)(use & 1), p.status, lane);
             ts_fence_after();
-            const int64_t n = c.group * TS_ROWS + r;
+            const int64_t n = group_of(c) * TS_ROWS + r;
             const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(d_col + buf * nb);
             const int slot = 2 * (int)blockIdx.x + (tile == first_tile ? 0 : 1);
             float *wsp = p.ws + (size_t)slot * nb * TS_ROWS + r;
@@ -432,7 +456,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                 ts_ld16(taddr + c0, v);
                 if (whole) {
                     if (n < p.N) {
-                        const int64_t at = (int64_t)(c.mb * nb + c0) * p.ldy + n;
+                        const int64_t at = (int64_t)(row0 + c0) * p.ldy + n;
 #pragma unroll
                         for (int i = 0; i < 16; i++)
                             if (c0 + i < rows) store_from_float(p.y, p.y_dt, at + i * p.ldy, __uint_as_float(v[i]) + bias);
@@ -460,7 +484,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             }
             left -= run;
             seg++;
-            c.advance(run, SBp, mbs);
+            c.advance(run, SBp, ni);
         }
     } else if (warp < TS_MMA_WARP) {
         // ---------------------------------------------------------------- expansion into tensor memory
@@ -468,14 +492,14 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32 + ((cw >> 2) & 1) * 16) << 16);
         int as = set, a_round = 0;  // A stage of the item, how often the stages have been filled before
         TsCursor c;
-        c.init(i0, SBp, mbs);
-        c.advance(set, SBp, mbs);
+        c.init(i0, SBp, ni);
+        c.advance(set, SBp, ni);
         bool alive = true;
         int s = 0;
         uint32_t rpar = 0;
         for (int k = 0; k < my_count; k++) {
             const uint32_t stage = my_ring + (uint32_t)(s * TB);
-            const bool have = c.group * TS_GROUP_TILES + tau < p.NT;
+            const bool have = group_of(c) * TS_GROUP_TILES + tau < p.NT;
             if (alive) alive = mbar_wait_bounded(my_bar + 8 * s, rpar, p.status);
             alive = __all_sync(0xffffffffu, alive);
             if (have) ts_header<FMT>(stage, hdr, lane);
@@ -494,7 +518,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                 as -= na;
                 a_round++;
             }
-            c.advance(2, SBp, mbs);
+            c.advance(2, SBp, ni);
             if (++s == ring) {
                 s = 0;
                 rpar ^= 1u;
@@ -558,19 +582,19 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         grid_dependency_wait();  // the images are written by the preceding kernel
         bool alive = true;
         TsCursor c;
-        c.init(i0, SBp, mbs);
+        c.init(i0, SBp, ni);
         const int64_t it_stride = ((int64_t)p.Mp >> 3) << 10;
         const uint8_t *img = reinterpret_cast<const uint8_t *>(p.xh);
         int slot = 0, filled = 0;
         uint32_t par = 1;
         for (int li = 0; li < n_items; li++) {
-            const uint8_t *from = img + (int64_t)c.sb * 4 * it_stride + (((int64_t)c.mb * nb >> 3) << 10);
+            const uint8_t *from = img + (int64_t)c.sb * 4 * it_stride + (((int64_t)row0_of(c) >> 3) << 10);
             for (int n = 0; n < 4; n += spb, filled++) {
                 if (filled >= bslots && alive) alive = __all_sync(0xffffffffu, ts_wait(b_empty + 8 * slot, par, p.status));
                 const uint32_t dst = b_u32 + (uint32_t)(slot * spb) * slice_bytes, bar = b_full + 8 * slot;
                 if (alive && ts_elect()) {
                     mbar_expect_tx(bar, spb * slice_bytes);
-                    if (mbs == 1) {
+                    if (p.Mp == nb) {
                         bulk_g2s(dst, from + n * it_stride, spb * slice_bytes, bar);  // the slices of one block are neighbours
                     } else {
                         for (int q = 0; q < spb; q++) bulk_g2s(dst + q * slice_bytes, from + (n + q) * it_stride, slice_bytes, bar);
@@ -581,7 +605,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                     par ^= 1u;
                 }
             }
-            c.advance(1, SBp, mbs);
+            c.advance(1, SBp, ni);
         }
     }
     ts_fence_before();
@@ -597,9 +621,10 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         if (tile < 0) continue;
         const int64_t c_first = ((tile * SBp + 1) * G - 1) / T;
         const int pieces = (int)(((tile + 1) * SBp * G - 1) / T - c_first) + 1;
-        const int64_t group = tile / mbs;
-        const int mb = (int)(tile - group * mbs);
-        const int rows = p.M - mb * nb < nb ? p.M - mb * nb : nb;
+        TsCursor c;
+        c.init(tile * SBp, SBp, ni);
+        const int64_t group = group_of(c);
+        const int rows = rows_of(c), row0 = row0_of(c);
         const size_t piece = (size_t)nb * TS_ROWS;
         // the first CTA of the tile parked its piece in its second slot, unless its own run starts inside the tile; every
         // other one in its first slot
@@ -612,16 +637,16 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             for (int c0 = 1; c0 < pieces; c0 += 6) {
                 float4 q[6];  // six pieces requested at once
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
-                    q[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (c0 + c < pieces) q[c] = __ldcg(reinterpret_cast<const float4 *>(w1 + (size_t)(2 * (c0 + c - 1)) * piece + at));
+                for (int z = 0; z < 6; z++) {
+                    q[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (c0 + z < pieces) q[z] = __ldcg(reinterpret_cast<const float4 *>(w1 + (size_t)(2 * (c0 + z - 1)) * piece + at));
                 }
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
-                    acc.x += q[c].x;
-                    acc.y += q[c].y;
-                    acc.z += q[c].z;
-                    acc.w += q[c].w;
+                for (int z = 0; z < 6; z++) {
+                    acc.x += q[z].x;
+                    acc.y += q[z].y;
+                    acc.z += q[z].z;
+                    acc.w += q[z].w;
                 }
             }
             const int64_t n = group * TS_ROWS + v4;
@@ -630,13 +655,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             for (int i = 0; i < 4; i++)
                 if (n + i < p.N) {
                     const float b = p.bias != nullptr ? load_as_float(p.bias, p.bias_dt, n + i) : 0.f;
-                    store_from_float(p.y, p.y_dt, (int64_t)(mb * nb + m) * p.ldy + n + i, o[i] + b);
+                    store_from_float(p.y, p.y_dt, (int64_t)(row0 + m) * p.ldy + n + i, o[i] + b);
                 }
         }
     }
 }
 
-template <int FMT>
+template <int FMT, bool GROUPED = false>
 cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
     constexpr int TB = tile_bytes(FMT);
     static bool configured[64] = {};  // per device: the shared-memory opt-in belongs to the device's copy of the function
@@ -645,7 +670,7 @@ cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(gemm_ts_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
+        e = cudaFuncSetAttribute(gemm_ts_kernel<FMT, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -660,7 +685,7 @@ cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
     if (p.bslots > TS_MAX_BSLOTS) p.bslots = TS_MAX_BSLOTS;
     if (p.bslots < 2) return cudaErrorNotSupported;
     const size_t smem = (size_t)fixed + (size_t)TS_CONV_WARPS * p.ring * TB + (size_t)p.bslots * p.spb * slice;
-    return launch_pdl(gemm_ts_kernel<FMT>, dim3((unsigned)grid), dim3(TS_THREADS), smem, st, p);
+    return launch_pdl(gemm_ts_kernel<FMT, GROUPED>, dim3((unsigned)grid), dim3(TS_THREADS), smem, st, p);
 }
 
 }  // namespace
@@ -690,6 +715,7 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     p.bias = a.bias; p.bias_dt = a.bias_dt;
     p.y = a.y; p.y_dt = a.y_dt; p.ldy = a.ldy;
     p.status = status;
+    p.group_tiles = nullptr; p.mt_group = nullptr; p.mt_row0 = nullptr; p.n_mt = nullptr; p.mt_cap = 0;
     cudaError_t e = launch_xh_images(a, p.Mp, Kp, xh, sms, fmt == TTQ_FMT_Q4_K ? 2 : (fmt == TTQ_FMT_Q6_K ? 3 : 4), st);
     if (e != cudaSuccess) return e;
     ++*launches;
@@ -698,6 +724,32 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     else e = ts_launch<TTQ_FMT_Q6_K>(p, grid, st);
     if (e == cudaSuccess) ++*launches;
     return e;
+}
+
+// Grouped form (Q4_K): row tile mt of the routed rows multiplies weight matrix mt_group[mt]; `xh` holds the images of the
+// routed rows in the slot order of this kernel.
+bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms) {
+    const int64_t groups = (g.N + TS_ROWS - 1) / TS_ROWS;
+    return g.ts_ws != nullptr && g.BM % 16 == 0 && g.BM <= 256 && groups * g.mt_cap <= g.ts_counters_cap &&
+           (size_t)2 * sms * g.BM * TS_ROWS * sizeof(float) <= g.ts_ws_bytes;
+}
+
+cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st) {
+    if (!gemm_ts_grouped_fits(g, sms)) return cudaErrorInvalidValue;
+    TsParams p;
+    p.nb = g.BM; p.mbs = 1;
+    p.M = (int)g.Mp; p.Mp = (int)g.Mp;
+    p.tiles = nullptr;
+    p.N = g.N; p.NT = g.NT; p.SBp = (int)g.SBp;
+    p.T = (g.N + TS_ROWS - 1) / TS_ROWS * g.SBp;
+    p.xh = xh;
+    p.ws = g.ts_ws;
+    p.counters = g.ts_counters;
+    p.bias = nullptr; p.bias_dt = TTQ_DT_F32;
+    p.y = g.y; p.y_dt = g.y_dt; p.ldy = g.ldy;
+    p.status = status;
+    p.group_tiles = g.group_tiles; p.mt_group = g.mt_group; p.mt_row0 = g.mt_row0; p.n_mt = g.n_mt; p.mt_cap = g.mt_cap;
+    return ts_launch<TTQ_FMT_Q4_K, true>(p, sms, st);
 }
 
 }  // namespace ttq

@@ -252,7 +252,15 @@ struct GroupedArgs {
     void *y;                            // [Mp][ldy] routed output rows
     int y_dt;
     int64_t ldy;
+    // tensor-memory kernel (ttq_gemm_ts.cu; BM any multiple of 16 up to 256): workspace for partial sums, arrival counters (zero
+    // between launches).  ts_ws == nullptr: the shared-memory GEMM.
+    float *ts_ws = nullptr;
+    size_t ts_ws_bytes = 0;
+    unsigned *ts_counters = nullptr;
+    int64_t ts_counters_cap = 0;
 };
+bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms);
+cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st);
 cudaError_t launch_gemm_grouped(const GroupedArgs &g, __half *xh, int sms, int *status, cudaStream_t st, int *launches);
 
 // Trellis-coded 3-bit format (ttq_tq3.cu); `packed` is the canonical buffer on the device.

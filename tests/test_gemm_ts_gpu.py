@@ -51,3 +51,23 @@ def test_rows_of_a_wider_matrix(ctx, fmt):
     ctx.check_device_status()
     assert torch.equal(out[:, :n], want) and not out[:, n:].any()
     lin.close()
+
+
+@pytest.mark.parametrize("t,n_exp,top_k", [(24, 32, 4), (9, 8, 8), (130, 8, 1), (250, 8, 4)])
+def test_grouped_row_tiles(ctx, t, n_exp, top_k):
+    """The expert layer at 16-, 32- and 128-row tiles: fewer items than CTAs, experts with more rows than a tile, every choice dropped."""
+    from test_moe_gpu import build, check, routing
+
+    hidden, inter = 1024, 768
+    layer, gu, dn = build(ctx, n_exp, hidden, inter, top_k, max_tokens=256, seed=n_exp + t)
+    ids, w = routing(t, n_exp, top_k, seed=t, skew=True)
+    got = check(ctx, layer, gu, dn, t, hidden, ids, w, seed=t)
+    none = check_dropped(ctx, layer, t, hidden, ids, w)
+    assert np.isfinite(got).all() and not none.any()
+    layer.close()
+
+
+def check_dropped(ctx, layer, t, hidden, ids, w):
+    y = layer.forward(make_x(t, hidden, 1).cuda(), torch.full(ids.shape, -1, dtype=torch.int32, device="cuda"), torch.from_numpy(w).cuda())
+    ctx.check_device_status()
+    return y.float().cpu().numpy()
