@@ -611,6 +611,20 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         if (e != cudaSuccess) return cuda_fail(ctx, e, "linear forward (GEMM) launch");
         return TTQ_OK;
     }
+    // Q8_0 / Q6_K, 5 to 8 rows: the integer decode kernel keeps four rows' planes in shared memory and reads those of a second pass
+    // from L2, row by row of weights; the exact form of the tensor-memory kernel does not care how many rows there are (4096 ->
+    // 28672, us: Q8_0 44 against 77, Q6_K 55 against 95; 4096 -> 128256 Q6_K 203 against 355).  From four items of 128 x 256
+    // weights per SM: below, its fixed cost does not pay (4096 -> 4096: 15.6 against 14.8 and 17.6 against 18.0).
+    if (M >= 5 && M <= 8 && !gated && use_gemm && gemm_supported(w->fmt) && w->fmt != TTQ_FMT_Q4_K &&
+        (w->N + 127) / 128 * w->SBp >= 4 * (int64_t)ctx->sms) {
+        a.x = x_dev; a.M = M; a.y = y_dev;
+        int launches = 0;
+        cudaError_t e = launch_gemm_ts_precise(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
+                                               ctx->split_counters_cap, st, &launches);
+        ctx->launches += launches;
+        if (e == cudaSuccess) return TTQ_OK;
+        if (e != cudaErrorNotSupported) return cuda_fail(ctx, e, "linear forward (tensor-memory decode) launch");
+    }
     // decode path; more rows than one pass holds are processed in groups of MAX_GEMV_M
     for (int64_t m0 = 0; m0 < M; m0 += MAX_GEMV_M) {
         a.x = reinterpret_cast<const uint8_t *>(x_dev) + (size_t)m0 * ldx * dt_size(x_dt);

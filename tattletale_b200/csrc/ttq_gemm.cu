@@ -175,32 +175,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[16]) {
 // divisions per slot, 2-byte loads of gated bf16 rows.  Projections of an 8B layer at 2048 rows: 989 -> 855 us.)
 // `early`: the whole grid is resident and fits beside the GEMM that follows, which may be set up right away.
 
-// K values 8 L .. 8 L + 7 of a super-block -> stage s (window) and 16-byte slot
-__device__ __forceinline__ void xh_place(int kmap, int L, int &s, int &slot) {
-    s = L & 3;
-    int q = L >> 2;  // kmap 0, 2: sub-block = slot, resp. 2 u + hi
-    if (kmap == 4) q = 2 * (q & 3) + (q >> 2);
-    if (kmap == 1 || kmap == 3) {
-        const int b = L >> 1;  // 16-wide sub-block 4 s' + 8 hi + u
-        s = 2 * ((b >> 2) & 1) + (L & 1);
-        q = 2 * (b & 3) + (b >> 3);
-    }
-    slot = kmap >= 2 ? ((q & 4) | ((q & 1) << 1) | ((q >> 1) & 1)) : q;
-}
-__device__ __forceinline__ void xh_unpack(const uint4 &raw, int dt, float (&v)[8]) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        if (dt == TTQ_DT_BF16) {
-            v[2 * q] = __uint_as_float(w[q] << 16);
-            v[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
-        } else {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
-            v[2 * q] = f.x;
-            v[2 * q + 1] = f.y;
-        }
-    }
-}
 template <bool GATED>
 __global__ void __launch_bounds__(256) xh_prep_kernel(const void *__restrict__ x, int x_dt, int64_t M, int64_t Mp, int64_t K,
                                                       int64_t Kp, int64_t ldx, __half *__restrict__ xh,

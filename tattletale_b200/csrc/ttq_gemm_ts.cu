@@ -22,6 +22,10 @@
 // pieces.  Measured (4096 -> 28672 / 14336 -> 4096 / 4096 -> 6144 / 4096 -> 4096, us; the shared-memory GEMM in brackets):
 // 17 rows 30.4 / 20.3 / 13.2 / 11.8 (65.3 / 41.8 / 27.0 / 18.9), 64 rows 35.4 / 27.6 / 16.2 / 15.1 (65.6 / 42.9 / 30.0 / 20.0), 128 rows 50.7 / 36.8 / 23.1 / 21.7
 // (68.9 / 45.9 / 34.4 / 22.7); Q8_0 and Q6_K, 4096 -> 28672, 12 rows: 31.7 (69.5) and 38.3 (78.2).
+//
+// Exact form (Q8_0, Q6_K, one block of 16 rows): every weight as its fp16 rounding plus the remainder, two products into the same
+// accumulator, activations exact after a power of two per row; half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 44 us,
+// Q6_K 55 (integer decode kernel: 77 and 95); error against 64 bits as the integer kernel's or below.
 #include "ttq_devutil.cuh"
 
 namespace ttq {
@@ -32,7 +36,11 @@ constexpr int TS_EPI_WARPS = 4, TS_CONV_WARPS = 16;
 constexpr int TS_MMA_WARP = TS_EPI_WARPS + TS_CONV_WARPS, TS_B_WARP = TS_MMA_WARP + 1;
 constexpr int TS_WARPS = TS_B_WARP + 1, TS_THREADS = TS_WARPS * 32;
 constexpr int TS_ROWS = 128, TS_GROUP_TILES = TS_ROWS / TILE_ROWS;
-constexpr int TS_HDR_ROW = 80, TS_HDR_BYTES = 16 * TS_HDR_ROW;  // per conversion warp: the scale records of its 16 rows
+// What a launch is: one matrix, many (mixture of experts), or one matrix with its weights as exact pairs of fp16 values.
+enum TsMode { TS_DENSE, TS_GROUPED, TS_PRECISE };
+// bytes of a row's scale record, and of a conversion warp's 16 records (the exact Q6_K form holds every scale as a pair)
+__host__ __device__ constexpr int ts_hdr_row(int fmt, int mode) { return mode == TS_PRECISE && fmt == TTQ_FMT_Q6_K ? 144 : 80; }
+__host__ __device__ constexpr int ts_hdr_bytes(int fmt, int mode) { return 16 * ts_hdr_row(fmt, mode); }
 constexpr int TS_MAX_RING = 4, TS_MAX_BSLOTS = 12;
 constexpr int TS_MAX_A = 3;  // A stages in tensor memory
 constexpr int TS_BAR_BYTES = (TS_CONV_WARPS * TS_MAX_RING + 2 * TS_MAX_BSLOTS + 2 * TS_MAX_A + 4) * 8 + 32;
@@ -63,6 +71,7 @@ struct TsParams {
     const uint8_t *const *group_tiles;
     const int *mt_group, *mt_row0, *n_mt;
     int64_t mt_cap;
+    const float *row_scale;  // exact form: the outputs of activation row m are multiplied by row_scale[m]
 };
 
 __device__ __forceinline__ void ts_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -138,8 +147,9 @@ __device__ __forceinline__ __half2 ts_as_h2(uint32_t v) { return *reinterpret_ca
 //   Q6_K  slice 2 s' + n = window n of sets s' (run 0) and s' + 2 (run 1)
 
 // Writes the scale records of the tile's 16 rows (lane (r, h): half h of row r).
-template <int FMT>
+template <int FMT, int MODE>
 __device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane) {
+    constexpr int TS_HDR_ROW = ts_hdr_row(FMT, MODE);
     const int r = lane & 15, h = lane >> 4;
     if constexpr (FMT == TTQ_FMT_Q4_K) {
         // sub-blocks 4h..4h+3: {scale, scale, offset, offset} halves, w = scale * (q - 8) + offset (high nibbles arrive as
@@ -185,11 +195,25 @@ __device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane
         const uint32_t dst = hdr + (uint32_t)(r * TS_HDR_ROW + h * 32);
         sts128<0>(dst, w[0], w[1], w[2], w[3]);
         sts128<16>(dst, w[4], w[5], w[6], w[7]);
+        if constexpr (MODE == TS_PRECISE) {
+            // what the rounding left out: d * sc has at most 19 significant bits
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float sc = d * (float)(int)(int8_t)(((i < 4 ? hv.x : hv.y) >> (8 * (i & 3))) & 0xff);
+                w[i] = ts_h2(__float2half2_rn(sc - __low2float(ts_as_h2(w[i]))));
+            }
+            sts128<64>(dst, w[0], w[1], w[2], w[3]);
+            sts128<80>(dst, w[4], w[5], w[6], w[7]);
+        }
     }
 }
 
-template <int FMT>
-__device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane, uint32_t taddr) {
+// PRECISE: two slices from slice n0 on, the rounded weights in columns 0..63 and what the rounding left out in columns 64..127
+// of the stage (w = q * scale: one fused multiply-add gives the remainder exactly); otherwise the four slices of the item.
+template <int FMT, int MODE>
+__device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane, uint32_t taddr, int n0) {
+    constexpr int TS_HDR_ROW = ts_hdr_row(FMT, MODE), SLICES = MODE == TS_PRECISE ? 2 : 4;
+    static_assert(MODE != TS_PRECISE || FMT != TTQ_FMT_Q4_K, "the exact form serves formats without an offset");
     // (the four slices are a loop, not unrolled: a quarter of the code to fetch at the start of every launch, and few enough
     // registers that the activation pass of the next linear can be resident beside this kernel)
     const int g = lane >> 2, t = lane & 3;
@@ -223,7 +247,7 @@ __device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane
         }
     } else if constexpr (FMT == TTQ_FMT_Q8_0) {
         const __half2 k1152 = __float2half2_rn(1152.f);
-        uint32_t s0[4], s1[4];
+        uint32_t s0[4], s1[4];  // scales of blocks u and 4 + u per register
         const uint32_t ha = hdr + (uint32_t)(g * TS_HDR_ROW + (t >> 1) * 4);
         s0[0] = lds32<0>(ha);
         s0[1] = lds32<8 * TS_HDR_ROW>(ha);
@@ -234,29 +258,36 @@ __device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane
         s1[2] = lds32<24>(ha);
         s1[3] = lds32<8 * TS_HDR_ROW + 24>(ha);
 #pragma unroll 1
-        for (int n = 0; n < 4; n++) {
+        for (int z = 0; z < SLICES; z++) {
+            const int n = n0 + z;
             const uint4 qa = lds128<0>(sa + n * 512), qb = lds128<2048>(sa + n * 512);
             const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w};
             const uint32_t wb[4] = {qb.x, qb.y, qb.z, qb.w};
-            uint32_t r[16];
+            uint32_t r[16], lo[16];
 #pragma unroll
             for (int sl = 0; sl < 4; sl++) {
                 // int8 -> fp16: flip the sign bit (q + 128 in 0..255), OR into the mantissa of 1024, subtract 1152
                 const int o = 8 * (sl >> 1) + 2 * (sl & 1);
                 const uint32_t x = wa[sl] ^ 0x80808080u, y = wb[sl] ^ 0x80808080u;
-                r[o + 0] = ts_h2(__hmul2(__hsub2(ts_as_h2(and_or(x, mask_b, k1024)), k1152), ts_as_h2(s0[sl])));
-                r[o + 1] = ts_h2(__hmul2(__hsub2(ts_as_h2(and_or(x >> 8, mask_b, k1024)), k1152), ts_as_h2(s0[sl])));
-                r[o + 4] = ts_h2(__hmul2(__hsub2(ts_as_h2(and_or(y, mask_b, k1024)), k1152), ts_as_h2(s1[sl])));
-                r[o + 5] = ts_h2(__hmul2(__hsub2(ts_as_h2(and_or(y >> 8, mask_b, k1024)), k1152), ts_as_h2(s1[sl])));
+                const uint32_t v[4] = {and_or(x, mask_b, k1024), and_or(x >> 8, mask_b, k1024), and_or(y, mask_b, k1024), and_or(y >> 8, mask_b, k1024)};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int at = o + (e & 1) + 4 * (e >> 1);
+                    const __half2 q = __hsub2(ts_as_h2(v[e]), k1152), sc = ts_as_h2(e < 2 ? s0[sl] : s1[sl]);
+                    const __half2 w = __hmul2(q, sc);
+                    r[at] = ts_h2(w);
+                    if constexpr (MODE == TS_PRECISE) lo[at] = ts_h2(__hfma2(q, sc, __hneg2(w)));
+                }
             }
-            ts_st_16x256b(taddr + n * 32, r);
+            ts_st_16x256b(taddr + z * 32, r);
+            if constexpr (MODE == TS_PRECISE) ts_st_16x256b(taddr + 64 + z * 32, lo);
         }
     } else {
         const __half2 k1056 = __float2half2_rn(1056.f);
 #pragma unroll 1
-        for (int n = 0; n < 4; n++) {
-            const int sp = n >> 1;  // set of the low nibbles; the high nibbles are set sp + 2
-            uint32_t s0[4], s1[4];
+        for (int z = 0; z < SLICES; z++) {
+            const int n = n0 + z, sp = n >> 1;  // set of the low nibbles; the high nibbles are set sp + 2
+            uint32_t s0[4], s1[4], t0[4], t1[4];
             const uint32_t ha = hdr + (uint32_t)(g * TS_HDR_ROW + (t >> 1) * 4 + sp * 16);
             s0[0] = lds32<0>(ha);
             s0[1] = lds32<8 * TS_HDR_ROW>(ha);
@@ -266,24 +297,40 @@ __device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane
             s1[1] = lds32<8 * TS_HDR_ROW + 32>(ha);
             s1[2] = lds32<40>(ha);
             s1[3] = lds32<8 * TS_HDR_ROW + 40>(ha);
+            if constexpr (MODE == TS_PRECISE) {
+                t0[0] = lds32<64>(ha);
+                t0[1] = lds32<8 * TS_HDR_ROW + 64>(ha);
+                t0[2] = lds32<72>(ha);
+                t0[3] = lds32<8 * TS_HDR_ROW + 72>(ha);
+                t1[0] = lds32<96>(ha);
+                t1[1] = lds32<8 * TS_HDR_ROW + 96>(ha);
+                t1[2] = lds32<104>(ha);
+                t1[3] = lds32<8 * TS_HDR_ROW + 104>(ha);
+            }
             const uint4 qa = lds128<0>(sa + n * 512), qb = lds128<2048>(sa + (n & 1) * 512);
             const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
-            uint32_t r[16];
+            uint32_t r[16], lo[16];
 #pragma unroll
             for (int sl = 0; sl < 4; sl++) {
                 // 6-bit quant = nibble | (two plane bits << 4); OR-ed into the mantissa of 1024, minus 1024 + 32
                 const int o = 8 * (sl >> 1) + 2 * (sl & 1);
                 const uint32_t x = wa[sl], x8 = x >> 8;
                 const uint32_t pl = wb[sl] >> (2 * sp), ph = wb[sl] >> (2 * sp + 4);
-                const uint32_t v0 = and_or(x, mask_lo, k1024) | ((pl << 4) & 0x00300030u), v1 = and_or(x8, mask_lo, k1024) | ((pl >> 4) & 0x00300030u);
-                const uint32_t v2 = and_or(x >> 4, mask_lo, k1024) | ((ph << 4) & 0x00300030u),
-                               v3 = and_or(x8 >> 4, mask_lo, k1024) | ((ph >> 4) & 0x00300030u);
-                r[o + 0] = ts_h2(__hmul2(__hsub2(ts_as_h2(v0), k1056), ts_as_h2(s0[sl])));
-                r[o + 1] = ts_h2(__hmul2(__hsub2(ts_as_h2(v1), k1056), ts_as_h2(s0[sl])));
-                r[o + 4] = ts_h2(__hmul2(__hsub2(ts_as_h2(v2), k1056), ts_as_h2(s1[sl])));
-                r[o + 5] = ts_h2(__hmul2(__hsub2(ts_as_h2(v3), k1056), ts_as_h2(s1[sl])));
+                const uint32_t v[4] = {and_or(x, mask_lo, k1024) | ((pl << 4) & 0x00300030u), and_or(x8, mask_lo, k1024) | ((pl >> 4) & 0x00300030u),
+                                       and_or(x >> 4, mask_lo, k1024) | ((ph << 4) & 0x00300030u),
+                                       and_or(x8 >> 4, mask_lo, k1024) | ((ph >> 4) & 0x00300030u)};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int at = o + (e & 1) + 4 * (e >> 1);
+                    const __half2 q = __hsub2(ts_as_h2(v[e]), k1056), sc = ts_as_h2(e < 2 ? s0[sl] : s1[sl]);
+                    const __half2 w = __hmul2(q, sc);
+                    r[at] = ts_h2(w);
+                    if constexpr (MODE == TS_PRECISE)
+                        lo[at] = ts_h2(__hfma2(q, ts_as_h2(e < 2 ? t0[sl] : t1[sl]), __hfma2(q, sc, __hneg2(w))));
+                }
             }
-            ts_st_16x256b(taddr + n * 32, r);
+            ts_st_16x256b(taddr + z * 32, r);
+            if constexpr (MODE == TS_PRECISE) ts_st_16x256b(taddr + 64 + z * 32, lo);
         }
     }
 }
@@ -311,10 +358,10 @@ struct TsCursor {
     }
 };
 
-// (GROUPED is a template parameter: the tables cost the registers that let the activation pass sit beside the dense form)
-template <int FMT, bool GROUPED>
+// (The mode is a template parameter: the tables cost the registers that let the activation pass sit beside the dense form)
+template <int FMT, int MODE>
 __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p) {
-    constexpr int TB = tile_bytes(FMT);
+    constexpr int TB = tile_bytes(FMT), TS_HDR_BYTES = ts_hdr_bytes(FMT, MODE);
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -331,7 +378,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     volatile int64_t *last_tile = reinterpret_cast<volatile int64_t *>(base_ptr + (d_empty + 32 - base));  // [2]
     // tensor memory: `na` stages of expanded weights, `nd` accumulator sets behind them
     const int na = nb <= 64 ? 3 : 2, nd = nb <= 128 ? 2 : 1, d_col = na * TS_A_COLS;
-    constexpr bool grouped = GROUPED;
+    constexpr bool grouped = MODE == TS_GROUPED, precise = MODE == TS_PRECISE;
     int64_t T = p.T;
     if (grouped) {
         grid_dependency_wait();  // the tables are written by preceding kernels
@@ -459,7 +506,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                         const int64_t at = (int64_t)(row0 + c0) * p.ldy + n;
 #pragma unroll
                         for (int i = 0; i < 16; i++)
-                            if (c0 + i < rows) store_from_float(p.y, p.y_dt, at + i * p.ldy, __uint_as_float(v[i]) + bias);
+                            if (c0 + i < rows) store_from_float(p.y, p.y_dt, at + i * p.ldy, __uint_as_float(v[i]) * (precise ? p.row_scale[c0 + i] : 1.f) + bias);
                     }
                 } else {
 #pragma unroll
@@ -490,7 +537,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         // ---------------------------------------------------------------- expansion into tensor memory
         const uint32_t hdr = hdr_u32 + (uint32_t)(cw * TS_HDR_BYTES);
         const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32 + ((cw >> 2) & 1) * 16) << 16);
-        int as = set, a_round = 0;  // A stage of the item, how often the stages have been filled before
+        int as = precise ? 2 * set : set, a_round = 0;  // A stage of the item, how often the stages have been filled before
         TsCursor c;
         c.init(i0, SBp, ni);
         c.advance(set, SBp, ni);
@@ -502,22 +549,28 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             const bool have = group_of(c) * TS_GROUP_TILES + tau < p.NT;
             if (alive) alive = mbar_wait_bounded(my_bar + 8 * s, rpar, p.status);
             alive = __all_sync(0xffffffffu, alive);
-            if (have) ts_header<FMT>(stage, hdr, lane);
+            if (have) ts_header<FMT, MODE>(stage, hdr, lane);
             __syncwarp();  // the records are written
-            if (a_round >= 1 && alive) alive = ts_wait_warp(a_empty + 8 * as, (uint32_t)((a_round - 1) & 1), p.status, lane);
-            ts_fence_after();
-            if (have) {
-                ts_expand<FMT>(stage, hdr, lane, taddr + (uint32_t)(as * TS_A_COLS));
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            // (exact form: the item takes two A stages, each two slices as rounded weights and remainders)
+#pragma unroll 1
+            for (int half = 0; half < (precise ? 2 : 1); half++) {
+                if (a_round >= 1 && alive) alive = ts_wait_warp(a_empty + 8 * as, (uint32_t)((a_round - 1) & 1), p.status, lane);
+                ts_fence_after();
+                if (have) {
+                    ts_expand<FMT, MODE>(stage, hdr, lane, taddr + (uint32_t)(as * TS_A_COLS), 2 * half);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                }
+                ts_fence_before();
+                __syncwarp();  // also: every lane has read the stage and the records
+                if (lane == 0) ts_arrive(a_full + 8 * as);
+                // the next stage of this set: two items on (dense); the item's second stage, then past the other set's two (exact)
+                as += precise ? (half == 0 ? 1 : 3) : 2;
+                while (as >= na) {
+                    as -= na;
+                    a_round++;
+                }
             }
-            ts_fence_before();
-            __syncwarp();  // also: every lane has read the stage and the records
-            if (lane == 0) ts_arrive(a_full + 8 * as);
             if (alive && issued < my_count) issue_next();
-            if ((as += 2) >= na) {
-                as -= na;
-                a_round++;
-            }
             c.advance(2, SBp, ni);
             if (++s == ring) {
                 s = 0;
@@ -532,42 +585,45 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         int sb = (int)(i0 - first_tile * SBp), seg = 0, slot = 0, as = 0;
         uint32_t bpar = 0, apar = 0;
         bool fresh = true;  // the next product starts an accumulator
+        const int step = precise ? 2 : spb;  // slices per hand-over (exact form: a whole item per activation slot, two A stages)
         for (int li = 0; li < n_items; li++) {
             const int buf = seg % nd, use = seg / nd;
             if (fresh && use >= 1 && alive) alive = ts_wait(d_empty + 8 * buf, (uint32_t)((use - 1) & 1), p.status);
-            if (alive) alive = ts_wait(a_full + 8 * as, apar, p.status);
             const uint32_t td = tmem_base + (uint32_t)(d_col + buf * nb);
             const bool done = sb + 1 == SBp || li == n_items - 1;
 #pragma unroll 1
-            for (int n = 0; n < 4; n += spb) {
-                if (alive) alive = ts_wait(b_full + 8 * slot, bpar, p.status);
+            for (int n = 0; n < 4; n += step) {
+                if ((precise || n == 0) && alive) alive = ts_wait(a_full + 8 * as, apar, p.status);
+                if ((!precise || n == 0) && alive) alive = ts_wait(b_full + 8 * slot, bpar, p.status);
                 __syncwarp();
                 ts_fence_after();
                 if (ts_elect()) {
-                    uint64_t bd = ts_desc_sw128(b_u32 + (uint32_t)(slot * spb) * slice_bytes);
-                    uint32_t ta = tmem_base + (uint32_t)(as * TS_A_COLS + n * 32);
-                    for (int q = 0; q < spb; q++) {
+                    uint64_t bd = ts_desc_sw128(b_u32 + (uint32_t)(slot * spb) * slice_bytes + (precise ? (uint32_t)n * slice_bytes : 0u));
+                    uint32_t ta = tmem_base + (uint32_t)(as * TS_A_COLS + (precise ? 0 : n * 32));
+                    for (int q = 0; q < step; q++) {
                         ts_mma(td, ta, bd, idesc, (fresh && n + q == 0) ? 0u : 1u);
 #pragma unroll
                         for (int kk = 1; kk < 4; kk++) ts_mma(td, ta + 8 * kk, bd + (uint64_t)(2 * kk), idesc, 1u);
+                        if (precise) {
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) ts_mma(td, ta + 64 + 8 * kk, bd + (uint64_t)(2 * kk), idesc, 1u);
+                        }
                         ta += 32;
                         bd += (uint64_t)(slice_bytes >> 4);
                     }
-                    ts_commit(b_empty + 8 * slot);
-                    if (n + spb == 4) {
-                        ts_commit(a_empty + 8 * as);
-                        if (done) ts_commit(d_full + 8 * buf);
-                    }
+                    if (!precise || n + step == 4) ts_commit(b_empty + 8 * slot);
+                    if (precise || n + step == 4) ts_commit(a_empty + 8 * as);
+                    if (n + step == 4 && done) ts_commit(d_full + 8 * buf);
                 }
                 __syncwarp();
-                if (++slot == bslots) {
+                if ((!precise || n + step == 4) && ++slot == bslots) {
                     slot = 0;
                     bpar ^= 1u;
                 }
-            }
-            if (++as == na) {
-                as = 0;
-                apar ^= 1u;
+                if ((precise || n + step == 4) && ++as == na) {
+                    as = 0;
+                    apar ^= 1u;
+                }
             }
             fresh = done;
             if (done) {
@@ -655,22 +711,22 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             for (int i = 0; i < 4; i++)
                 if (n + i < p.N) {
                     const float b = p.bias != nullptr ? load_as_float(p.bias, p.bias_dt, n + i) : 0.f;
-                    store_from_float(p.y, p.y_dt, (int64_t)(row0 + m) * p.ldy + n + i, o[i] + b);
+                    store_from_float(p.y, p.y_dt, (int64_t)(row0 + m) * p.ldy + n + i, o[i] * (precise ? p.row_scale[m] : 1.f) + b);
                 }
         }
     }
 }
 
-template <int FMT, bool GROUPED = false>
+template <int FMT, int MODE = TS_DENSE>
 cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
-    constexpr int TB = tile_bytes(FMT);
+    constexpr int TB = tile_bytes(FMT), TS_HDR_BYTES = ts_hdr_bytes(FMT, MODE);
     static bool configured[64] = {};  // per device: the shared-memory opt-in belongs to the device's copy of the function
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(gemm_ts_kernel<FMT, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
+        e = cudaFuncSetAttribute(gemm_ts_kernel<FMT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -683,9 +739,9 @@ cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
     p.spb = room >= 12 * slice ? 4 : (room >= 6 * slice ? 2 : 1);
     p.bslots = room / (slice * p.spb);
     if (p.bslots > TS_MAX_BSLOTS) p.bslots = TS_MAX_BSLOTS;
-    if (p.bslots < 2) return cudaErrorNotSupported;
+    if (p.bslots < 2 || (MODE == TS_PRECISE && p.spb != 4)) return cudaErrorNotSupported;
     const size_t smem = (size_t)fixed + (size_t)TS_CONV_WARPS * p.ring * TB + (size_t)p.bslots * p.spb * slice;
-    return launch_pdl(gemm_ts_kernel<FMT, GROUPED>, dim3((unsigned)grid), dim3(TS_THREADS), smem, st, p);
+    return launch_pdl(gemm_ts_kernel<FMT, MODE>, dim3((unsigned)grid), dim3(TS_THREADS), smem, st, p);
 }
 
 }  // namespace
@@ -715,6 +771,7 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     p.bias = a.bias; p.bias_dt = a.bias_dt;
     p.y = a.y; p.y_dt = a.y_dt; p.ldy = a.ldy;
     p.status = status;
+    p.row_scale = nullptr;
     p.group_tiles = nullptr; p.mt_group = nullptr; p.mt_row0 = nullptr; p.n_mt = nullptr; p.mt_cap = 0;
     cudaError_t e = launch_xh_images(a, p.Mp, Kp, xh, sms, fmt == TTQ_FMT_Q4_K ? 2 : (fmt == TTQ_FMT_Q6_K ? 3 : 4), st);
     if (e != cudaSuccess) return e;
@@ -722,6 +779,96 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     if (fmt == TTQ_FMT_Q4_K) e = ts_launch<TTQ_FMT_Q4_K>(p, grid, st);
     else if (fmt == TTQ_FMT_Q8_0) e = ts_launch<TTQ_FMT_Q8_0>(p, grid, st);
     else e = ts_launch<TTQ_FMT_Q6_K>(p, grid, st);
+    if (e == cudaSuccess) ++*launches;
+    return e;
+}
+
+namespace {
+
+// Rows of the exact form: every row is brought by a power of two to a largest magnitude in [512, 1024), where a bf16 or f16
+// value is exact in fp16 down to 2^-24 of 512; `scale[m]` undoes it.  One CTA per image row (rows beyond M: zeros).
+__global__ void __launch_bounds__(512) xh_rows_kernel(const void *__restrict__ x, int x_dt, int M, int64_t K, int64_t Kp, int64_t ldx,
+                                                      __half *__restrict__ xh, float *__restrict__ scale, int kmap) {
+    __shared__ float red[16];
+    grid_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = blockIdx.x;
+    const int SBp = (int)(Kp >> 8);
+    int s, slot;
+    xh_place(kmap, lane, s, slot);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ldx * 2)) & 15) == 0;
+    grid_dependency_wait();
+    auto load = [&](int sb, float (&v)[8]) {
+        const int64_t k0 = (int64_t)sb * 256 + 8 * lane;
+        if (m < M && aligned && k0 + 8 <= K) {
+            xh_unpack(*reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(x) + m * ldx + k0), x_dt, v);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = m < M && k0 + i < K ? load_as_float(x, x_dt, m * ldx + k0 + i) : 0.f;
+        }
+    };
+    float v[8], amax = 0.f;
+    for (int sb = warp; sb < SBp; sb += 16) {
+        load(sb, v);
+#pragma unroll
+        for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red[warp] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 16; w++) amax = fmaxf(amax, red[w]);
+    // (two factors, so that neither leaves the range of a float: |9 - e| is at most 158)
+    const int e = amax > 0.f && amax < 3.0e38f ? 9 - ilogbf(amax) : 0, e1 = e / 2, e2 = e - e1;
+    const float f1 = ldexpf(1.f, e1), f2 = ldexpf(1.f, e2);
+    if (threadIdx.x == 0) scale[m] = ldexpf(1.f, -e);
+    for (int sb = warp; sb < SBp; sb += 16) {
+        load(sb, v);
+        uint32_t o[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int a = (q >> 1) * 4 + (q & 1);
+            o[q] = ts_h2(__floats2half2_rn(v[a] * f1 * f2, v[a + 2] * f1 * f2));
+        }
+        const int64_t it = (int64_t)sb * 4 + s;
+        const int64_t dst = ((it * (gridDim.x >> 3) + (m >> 3)) << 10) + ((m & 7) << 7) + ((slot ^ (m & 7)) << 4);
+        *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xh) + dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+}  // namespace
+
+// Q8_0 / Q6_K, up to 16 rows, with weights and activations exact: the accuracy of the integer decode kernel at the rate of
+// the tensor cores.  Not for the gated form, whose products would be rounded to fp16.
+cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
+                                   int64_t counters_cap, cudaStream_t st, int *launches) {
+    *launches = 0;
+    constexpr int NB = 16;
+    if ((fmt != TTQ_FMT_Q8_0 && fmt != TTQ_FMT_Q6_K) || a.M < 1 || a.M > NB || a.gated) return cudaErrorNotSupported;
+    TsParams p;
+    p.mbs = 1; p.nb = NB;
+    p.M = (int)a.M; p.Mp = NB;
+    p.tiles = a.tiles;
+    p.N = a.N; p.NT = a.NT; p.SBp = (int)a.SBp;
+    const int64_t groups = (a.N + TS_ROWS - 1) / TS_ROWS;
+    p.T = groups * a.SBp;
+    const int grid = (int)(p.T < sms ? p.T : sms);
+    const int64_t Kp = a.SBp * TILE_K;
+    const size_t xh_bytes = (size_t)NB * Kp * sizeof(__half), ws_at = xh_bytes + 256;  // 256: the row scales
+    if (ws_at + (size_t)2 * grid * NB * TS_ROWS * sizeof(float) > (size_t)xh_capacity * sizeof(__half) || groups > counters_cap) return cudaErrorNotSupported;
+    float *scale = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + xh_bytes);
+    p.xh = xh;
+    p.ws = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + ws_at);
+    p.row_scale = scale;
+    p.counters = counters;
+    p.bias = a.bias; p.bias_dt = a.bias_dt;
+    p.y = a.y; p.y_dt = a.y_dt; p.ldy = a.ldy;
+    p.status = status;
+    p.group_tiles = nullptr; p.mt_group = nullptr; p.mt_row0 = nullptr; p.n_mt = nullptr; p.mt_cap = 0;
+    cudaError_t e = launch_pdl(xh_rows_kernel, dim3(NB), dim3(512), 0, st, a.x, a.x_dt, (int)a.M, a.K, Kp, a.ldx, xh, scale, fmt == TTQ_FMT_Q6_K ? 3 : 4);
+    if (e != cudaSuccess) return e;
+    ++*launches;
+    e = fmt == TTQ_FMT_Q8_0 ? ts_launch<TTQ_FMT_Q8_0, TS_PRECISE>(p, grid, st) : ts_launch<TTQ_FMT_Q6_K, TS_PRECISE>(p, grid, st);
     if (e == cudaSuccess) ++*launches;
     return e;
 }
@@ -748,8 +895,9 @@ cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int s
     p.bias = nullptr; p.bias_dt = TTQ_DT_F32;
     p.y = g.y; p.y_dt = g.y_dt; p.ldy = g.ldy;
     p.status = status;
+    p.row_scale = nullptr;
     p.group_tiles = g.group_tiles; p.mt_group = g.mt_group; p.mt_row0 = g.mt_row0; p.n_mt = g.n_mt; p.mt_cap = g.mt_cap;
-    return ts_launch<TTQ_FMT_Q4_K, true>(p, sms, st);
+    return ts_launch<TTQ_FMT_Q4_K, TS_GROUPED>(p, sms, st);
 }
 
 }  // namespace ttq

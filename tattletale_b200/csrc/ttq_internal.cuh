@@ -259,6 +259,8 @@ struct GroupedArgs {
     unsigned *ts_counters = nullptr;
     int64_t ts_counters_cap = 0;
 };
+cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
+                                   int64_t counters_cap, cudaStream_t st, int *launches);
 bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms);
 cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st);
 cudaError_t launch_gemm_grouped(const GroupedArgs &g, __half *xh, int sms, int *status, cudaStream_t st, int *launches);
@@ -349,6 +351,34 @@ __device__ __forceinline__ void store_from_float(void *p, int dt, int64_t i, flo
     if (dt == TTQ_DT_BF16) reinterpret_cast<__nv_bfloat16 *>(p)[i] = __float2bfloat16_rn(v);
     else if (dt == TTQ_DT_F16) reinterpret_cast<__half *>(p)[i] = __float2half_rn(v);
     else reinterpret_cast<float *>(p)[i] = v;
+}
+
+// ---- activation images of the tensor-core kernels (layout: xh_prep_kernel, ttq_gemm.cu) ----
+// K values 8 L .. 8 L + 7 of a super-block -> stage s (window) and 16-byte slot
+__device__ __forceinline__ void xh_place(int kmap, int L, int &s, int &slot) {
+    s = L & 3;
+    int q = L >> 2;  // kmap 0, 2: sub-block = slot, resp. 2 u + hi
+    if (kmap == 4) q = 2 * (q & 3) + (q >> 2);
+    if (kmap == 1 || kmap == 3) {
+        const int b = L >> 1;  // 16-wide sub-block 4 s' + 8 hi + u
+        s = 2 * ((b >> 2) & 1) + (L & 1);
+        q = 2 * (b & 3) + (b >> 3);
+    }
+    slot = kmap >= 2 ? ((q & 4) | ((q & 1) << 1) | ((q >> 1) & 1)) : q;
+}
+__device__ __forceinline__ void xh_unpack(const uint4 &raw, int dt, float (&v)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if (dt == TTQ_DT_BF16) {
+            v[2 * q] = __uint_as_float(w[q] << 16);
+            v[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
+            v[2 * q] = f.x;
+            v[2 * q + 1] = f.y;
+        }
+    }
 }
 
 // (a & b) | c in one instruction with both constants in registers (written with immediates the compiler emits

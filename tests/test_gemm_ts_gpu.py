@@ -71,3 +71,27 @@ def check_dropped(ctx, layer, t, hidden, ids, w):
     y = layer.forward(make_x(t, hidden, 1).cuda(), torch.full(ids.shape, -1, dtype=torch.int32, device="cuda"), torch.from_numpy(w).cuda())
     ctx.check_device_status()
     return y.float().cpu().numpy()
+
+
+@pytest.mark.parametrize("fmt", [ttq.FMT_Q8_0, ttq.FMT_Q6_K], ids=["q8_0", "q6_k"])
+@pytest.mark.parametrize("n,k,m", [(76800, 256, 5), (9500, 2048, 8), (4130, 4608, 6), (2000, 9984, 7)])
+def test_exact_form_of_five_to_eight_rows(ctx, fmt, n, k, m):
+    """Weights as pairs of fp16 values (remainder below 2^-22 of the weight), activations exact after a power of two: what is left is
+    the fp32 accumulation; bar 3e-5, the error of the integer decode kernel's 16-bit fixed point.  A power of two on a row
+    multiplies its outputs by exactly that, far outside the range of fp16."""
+    dtype = torch.float16 if m % 2 else torch.bfloat16
+    blocks = make_weight(fmt, n, k, seed=n + k + m)
+    x = make_x(m, k, seed=m + 1, dtype=dtype)
+    bias = torch.from_numpy(np.random.default_rng(m).normal(0, 0.1, n).astype(np.float32))
+    lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks), k, bias=bias.cuda())
+    y = lin.forward(x.cuda(), out_dtype=torch.float32)
+    want = oracle.linear(OFMT[fmt], blocks, x_bits(x), odt(dtype), bias.numpy())
+    assert rel_l2(y.cpu().numpy(), want) < 3e-5
+    wide = x.to(torch.bfloat16).cuda()
+    factor = torch.ones(m, 1, device="cuda")
+    factor[0], factor[1], factor[m - 1] = 2.0 ** 60, 2.0 ** -60, 0.0
+    plain = lin.forward(wide, out_dtype=torch.float32, use_bias=False)
+    scaled = lin.forward((wide * factor).to(torch.bfloat16), out_dtype=torch.float32, use_bias=False)
+    ctx.check_device_status()
+    assert torch.equal(scaled, plain * factor)
+    lin.close()
