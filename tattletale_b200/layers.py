@@ -371,7 +371,10 @@ class GatedMLP:
         gate_up = self.gate_up_proj.forward(x)
         if self.activation != ActivationKind.kSilu:
             raise TtqError(3, f"activation {self.activation} is not implemented")
-        return self.down_proj.forward(silu_and_mul(self.ctx, gate_up))
+        if self.down_proj.fmt == _lib.FMT_TQ3:
+            return self.down_proj.forward(silu_and_mul(self.ctx, gate_up))
+        # the activation inside the down projection's input conversion: one pass over gate|up and one rounding less
+        return self.down_proj.forward_gated(gate_up)
 
     __call__ = forward
 
