@@ -595,11 +595,10 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         // prefill / larger batches: tensor-core path
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
-        // Up to 192 rows the tensor-memory kernel (4096 -> 28672, us, it against the shared-memory GEMM: 30 / 65 at 17 rows, 51 / 69
-        // at 128, 75 / 81 at 192); up to 256 while there are fewer 128-row groups of weights than SMs, where its even split of K
-        // wins (4096 -> 6144 at 256 rows 38 / 46, 14336 -> 4096 54 / 58; 4096 -> 28672: 85 / 82).  Beyond, every block of rows would
-        // expand the weights again.
-        if (M <= 192 || (M <= 256 && w->N <= (int64_t)128 * ctx->sms)) {
+        // Up to 256 rows the tensor-memory kernel (4096 -> 28672, us, it against the shared-memory GEMM: 30 / 65 at 17 rows, 49 / 69 at
+        // 112, 78 / 82 at 256; 4096 -> 6144 at 256 rows 39 / 46), for Q8_0 with more 128-row groups of weights than SMs up to 192 (at
+        // 256 rows 95 / 86).  Beyond, every further block of rows would expand the weights again.
+        if (M <= 192 || (M <= 256 && (w->fmt != TTQ_FMT_Q8_0 || w->N <= (int64_t)128 * ctx->sms))) {
             cudaError_t e = launch_gemm_ts(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
                                            ctx->split_counters_cap, st, &launches);
             ctx->launches += launches;

@@ -706,13 +706,35 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                 }
             }
             const int64_t n = group * TS_ROWS + v4;
-            const float o[4] = {acc.x, acc.y, acc.z, acc.w};
+            float o[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (n + i < p.N) {
-                    const float b = p.bias != nullptr ? load_as_float(p.bias, p.bias_dt, n + i) : 0.f;
-                    store_from_float(p.y, p.y_dt, (int64_t)(row0 + m) * p.ldy + n + i, o[i] * (precise ? p.row_scale[m] : 1.f) + b);
+            for (int i = 0; i < 4; i++) {
+                if (precise) o[i] *= p.row_scale[m];
+                if (p.bias != nullptr && n + i < p.N) o[i] += load_as_float(p.bias, p.bias_dt, n + i);
+            }
+            // four outputs in one store where they lie so (y may be host memory, where every store is a transfer of its own)
+            const int64_t yi = (int64_t)(row0 + m) * p.ldy + n;
+            uint8_t *yp = reinterpret_cast<uint8_t *>(p.y) + yi * (p.y_dt == TTQ_DT_F32 ? 4 : 2);
+            const bool whole4 = n + 4 <= p.N;
+            if (whole4 && p.y_dt == TTQ_DT_F32 && (reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
+                *reinterpret_cast<float4 *>(yp) = make_float4(o[0], o[1], o[2], o[3]);
+            } else if (whole4 && p.y_dt != TTQ_DT_F32 && (reinterpret_cast<uintptr_t>(yp) & 7) == 0) {
+                uint32_t w[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    if (p.y_dt == TTQ_DT_BF16) {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+                        w[i] = *reinterpret_cast<const uint32_t *>(&h);
+                    } else {
+                        w[i] = ts_h2(__floats2half2_rn(o[2 * i], o[2 * i + 1]));
+                    }
                 }
+                *reinterpret_cast<uint2 *>(yp) = make_uint2(w[0], w[1]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (n + i < p.N) store_from_float(p.y, p.y_dt, yi + i, o[i]);
+            }
         }
     }
 }
@@ -730,10 +752,11 @@ cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
-    // Three ring stages of packed tiles cover the memory latency; with wide blocks the tensor cores set the pace, two do and
-    // the room goes to the activations.  A slot is a whole item while at least three of them fit.
+    // Three ring stages of packed tiles cover the memory latency of narrow blocks.  From 80 rows the activation slices (latency times
+    // rate out of L2) set the pace: two stages do, and the room holds more slices (4096 -> 28672 at 80 rows 44.7 -> 37.7 us, at 137
+    // rows 71.3 -> 56.8).  A slot is a whole item while at least three of them fit.
     const int fixed = 1024 + TS_CONV_WARPS * TS_HDR_BYTES + TS_BAR_BYTES, slice = p.nb * 128;
-    p.ring = 3;
+    p.ring = p.nb > 64 ? 2 : 3;
     while (p.ring > 2 && fixed + TS_CONV_WARPS * p.ring * TB + 4 * slice > TS_SMEM_MAX) p.ring--;
     const int room = TS_SMEM_MAX - fixed - TS_CONV_WARPS * p.ring * TB;
     p.spb = room >= 12 * slice ? 4 : (room >= 6 * slice ? 2 : 1);
