@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
         }
     } else if (PLAIN && warp < GEMM_EPI_WARPS + C::DEQ_WARPS) {
         // ------------------------------------------------------------------ producer: both operands are bulk copies
-        if (warp == GEMM_EPI_WARPS && lane == 0) {
+        if (warp == GEMM_EPI_WARPS) {
             grid_dependency_wait();  // both operands are written by preceding kernels
             bool alive = true;
             int git = 0;
@@ -465,11 +465,14 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (git >= STAGES && alive)
-                        alive = mbar_wait_bounded(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status);
+                        alive = __all_sync(0xffffffffu, mbar_wait_bounded(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status));
                     const uint32_t a_stage = stages_u32 + stage * C::STAGE_BYTES;
-                    mbar_expect_tx(full_bar + 8 * stage, C::A_BYTES + C::B_BYTES);
-                    bulk_g2s(a_stage, wsrc0 + it * w_it_stride, C::A_BYTES, full_bar + 8 * stage);
-                    bulk_g2s(a_stage + C::A_BYTES, bsrc0 + it * b_it_stride, C::B_BYTES, full_bar + 8 * stage);
+                    __syncwarp();
+                    if (elect_one()) {
+                        mbar_expect_tx(full_bar + 8 * stage, C::A_BYTES + C::B_BYTES);
+                        bulk_g2s(a_stage, wsrc0 + it * w_it_stride, C::A_BYTES, full_bar + 8 * stage);
+                        bulk_g2s(a_stage + C::A_BYTES, bsrc0 + it * b_it_stride, C::B_BYTES, full_bar + 8 * stage);
+                    }
                 }
             }
         }
@@ -1272,19 +1275,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
 }
 
 // Sum of the split-K partials (+ bias) into y.
-// A CTA takes 1024 columns of one row at a time, a thread four neighbours (16-byte loads of every partial where N is a multiple
-// of four; the partials are read once, from L2 as long as they fit).
+// A thread adds four neighbouring columns (16-byte loads of every partial where N is a multiple of four).
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ ws, int splits, int64_t M, int64_t Mp, int64_t N,
                                                             const void *bias, int bias_dt, void *y, int y_dt, int64_t ldy) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const uint32_t pieces = (uint32_t)((N + 1023) / 1024);
-    const uint32_t total = (uint32_t)M * pieces;
+    const uint32_t n4 = (uint32_t)((N + 3) / 4), total = (uint32_t)M * n4;  // (a slab has at most 64 MB of activations: M * N / 4 fits)
     const bool vec = (N & 3) == 0;
-    for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
-        const uint32_t m = b / pieces;
-        const int64_t n = (int64_t)(b - m * pieces) * 1024 + 4 * threadIdx.x;
-        if (n >= N) continue;
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < total; b += gridDim.x * blockDim.x) {
+        const uint32_t m = b / n4;
+        const int64_t n = (int64_t)(b - m * n4) * 4;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         if (vec) {
             for (int s = 0; s < splits; s++) {
@@ -1383,8 +1383,9 @@ cudaError_t launch_pair(const GemmParams &p, int sms, cudaStream_t st) {
 
 // Time of the pair kernel over `cols` weight-tile columns, in pipeline stages of the one-CTA kernel: the load of the first
 // pair, tiles dealt round-robin, full tiles (512 rows) before half tiles (256 rows).
-double pair_makespan(int64_t cols, int64_t m_full, int64_t m_half, int64_t slots, double iters) {
-    const double c_full = 0.73 * iters + 8.0, c_half = 0.52 * iters + 6.0;
+// `aligned`: output rows start on 16-byte boundaries; if not, the drain that nothing overlaps goes out in 2-byte pieces.
+double pair_makespan(int64_t cols, int64_t m_full, int64_t m_half, int64_t slots, double iters, bool aligned) {
+    const double c_full = (aligned ? 0.73 : 0.85) * iters + 8.0, c_half = (aligned ? 0.52 : 0.6) * iters + 6.0;
     const int64_t nf = cols * m_full, nt = nf + cols * m_half;
     double t = 0;
     for (int64_t k = 0; slots > 0 && k < nt; k += slots) t += k < nf ? c_full : c_half;
@@ -1439,10 +1440,11 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
     if (force_nsub == 1 || force_nsub == 2) nsub = force_nsub;
     // (the pair kernel's tiles are two sub-tiles wide: where a single sub-tile would only spare the one-CTA kernel a ragged round,
     // the pair may still be the cheaper one -- 4096 -> 6144 at 2048 rows: 110 against 136 us)
-    if (nsub == 1 && pair_mode > 0 && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && a.N > 128 && force_nsub == 0) {
+    const bool y_aligned = ((reinterpret_cast<uintptr_t>(a.y) | (uintptr_t)(a.ldy * (a.y_dt == TTQ_DT_F32 ? 4 : 2))) & 15) == 0;
+    if (nsub == 1 && pair_mode > 0 && y_aligned && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && a.N > 128 && force_nsub == 0) {
         const double iters = (double)a.SBp * 4;
         const int64_t slots = pair_slots(sms), mp = mt * 256;
-        if (slots > 0 && tiles2 > sms / 2 && pair_makespan((a.N + 255) / 256, mp / 512, mp % 512 ? 1 : 0, slots, iters) < cost1 * (iters + 8.0) / 1.65)
+        if (slots > 0 && tiles2 > sms / 2 && pair_makespan((a.N + 255) / 256, mp / 512, mp % 512 ? 1 : 0, slots, iters, true) < cost1 * (iters + 8.0) / 1.65)
             nsub = 2;
     }
     if (plain || fmt != TTQ_FMT_Q4_K) nsub = 2;  // plain: no conversion work to balance; Q8_0 / Q6_K: one variant
@@ -1519,7 +1521,7 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
             return launch_cfg<256, 1>(q, sms, st);
         };
         auto reduce = [&](const GemmParams &q) -> cudaError_t {
-            const int64_t total = Ms * ((q.N + 1023) / 1024);
+            const int64_t total = (Ms * ((q.N + 3) / 4) + 255) / 256;
             const unsigned rg = (unsigned)(total < sms * 8 ? total : sms * 8);
             return launch_pdl(splitk_reduce_kernel, dim3(rg), dim3(256), 0, st, (const float *)q.ws, q.splits, Ms, Mp, q.N, q.bias, q.bias_dt,
                               (void *)q.y, q.y_dt, q.ldy);
@@ -1575,7 +1577,7 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
         bool use_pair = false;
         if (pair_mode > 0 && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && nsub == 2 && splits == 1) {
             const int64_t slots = pair_slots(sms), m_full = Mp / 512, m_half = (Mp % 512) ? 1 : 0;
-            auto makespan = [&](int64_t cols) { return pair_makespan(cols, m_full, m_half, slots, iters); };
+            auto makespan = [&](int64_t cols) { return pair_makespan(cols, m_full, m_half, slots, iters, y_aligned); };
             double best = makespan(n_tiles);
             int64_t best_cols = 0;
             int best_runs = 1;
