@@ -595,10 +595,14 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         // prefill / larger batches: tensor-core path
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
-        // Up to 256 rows the tensor-memory kernel (4096 -> 28672, us, it against the shared-memory GEMM: 30 / 65 at 17 rows, 49 / 69 at
-        // 112, 78 / 82 at 256; 4096 -> 6144 at 256 rows 39 / 46), for Q8_0 with more 128-row groups of weights than SMs up to 192 (at
-        // 256 rows 95 / 86).  Beyond, every further block of rows would expand the weights again.
-        if (M <= 192 || (M <= 256 && (w->fmt != TTQ_FMT_Q8_0 || w->N <= (int64_t)128 * ctx->sms))) {
+        // Up to 192 rows the tensor-memory kernel (4096 -> 28672, us, it against the shared-memory GEMM: 30 / 65 at 17 rows, 49 / 69 at
+        // 112, 78 / 82 at 192; 4096 -> 1024 at 128 rows 20 / 22).  Up to 256 where there is more than a little work and fewer 128-row
+        // groups of weights than SMs (at 256 rows 4096 -> 6144 39 / 46, 12032 -> 1500 43 / 132), not where the sum of the pieces shows
+        // (4096 -> 1024 at 250 rows 32 / 24, 4096 -> 4096 at 256 rows 35 / 28) or the shared-memory GEMM fills its rounds (4096 ->
+        // 28672 at 256 rows 85 / 82, Q8_0 95 / 86).  Beyond, every further block of rows would expand the weights again.
+        const int64_t groups = (w->N + 127) / 128;
+        const bool large = groups * w->SBp >= 5 * (int64_t)ctx->sms || w->SBp >= 32;
+        if (M <= 192 || (M <= 256 && large && groups <= ctx->sms)) {
             cudaError_t e = launch_gemm_ts(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
                                            ctx->split_counters_cap, st, &launches);
             ctx->launches += launches;

@@ -26,6 +26,8 @@
 // Exact form (Q8_0, Q6_K, one block of 16 rows): every weight as its fp16 rounding plus the remainder, two products into the same
 // accumulator, activations exact after a power of two per row; half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 44 us,
 // Q6_K 55 (integer decode kernel: 77 and 95); error against 64 bits as the integer kernel's or below.
+#include <cmath>
+
 #include "ttq_devutil.cuh"
 
 namespace ttq {
@@ -739,6 +741,16 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     }
 }
 
+// CTAs of a dense launch.  One per SM, unless that cuts a tile into so many pieces that the CTA that adds them up works longer
+// than the cut saves: an item takes about 0.9 + 0.0055 nb us, a piece nb / 160 us in that CTA, and a tile of SBp items in c pieces
+// SBp / c items and c pieces.
+int ts_grid(int64_t T, int64_t tiles, int SBp, int nb, int sms) {
+    int64_t g = T < sms ? T : sms;
+    const double c = sqrt((double)SBp * (0.9 + 0.0055 * nb) * 160.0 / nb);
+    const int64_t most = (int64_t)((double)tiles * (c < 1.0 ? 1.0 : c));
+    return (int)(g < most ? g : most);
+}
+
 template <int FMT, int MODE = TS_DENSE>
 cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
     constexpr int TB = tile_bytes(FMT), TS_HDR_BYTES = ts_hdr_bytes(FMT, MODE);
@@ -783,7 +795,7 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     p.N = a.N; p.NT = a.NT; p.SBp = (int)a.SBp;
     const int64_t groups = (a.N + TS_ROWS - 1) / TS_ROWS;
     p.T = groups * p.mbs * a.SBp;
-    const int grid = (int)(p.T < sms ? p.T : sms);
+    const int grid = ts_grid(p.T, groups * p.mbs, p.SBp, p.nb, sms);
     const int64_t Kp = a.SBp * TILE_K;
     const size_t xh_bytes = ((size_t)p.Mp * Kp * sizeof(__half) + 255) & ~(size_t)255;
     const size_t ws_bytes = (size_t)2 * grid * p.nb * TS_ROWS * sizeof(float);
@@ -875,7 +887,7 @@ cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int
     p.N = a.N; p.NT = a.NT; p.SBp = (int)a.SBp;
     const int64_t groups = (a.N + TS_ROWS - 1) / TS_ROWS;
     p.T = groups * a.SBp;
-    const int grid = (int)(p.T < sms ? p.T : sms);
+    const int grid = ts_grid(p.T, groups, p.SBp, NB, sms);
     const int64_t Kp = a.SBp * TILE_K;
     const size_t xh_bytes = (size_t)NB * Kp * sizeof(__half), ws_at = xh_bytes + 256;  // 256: the row scales
     if (ws_at + (size_t)2 * grid * NB * TS_ROWS * sizeof(float) > (size_t)xh_capacity * sizeof(__half) || groups > counters_cap) return cudaErrorNotSupported;
