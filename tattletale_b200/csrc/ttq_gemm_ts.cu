@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(512) xh_rows_kernel(const void *__restrict__ x
 #pragma unroll
     for (int w = 0; w < 16; w++) amax = fmaxf(amax, red[w]);
     // (two factors, so that neither leaves the range of a float: |9 - e| is at most 158)
-    const int e = amax > 0.f && amax < 3.0e38f ? 9 - ilogbf(amax) : 0, e1 = e / 2, e2 = e - e1;
+    const int e = amax > 0.f && isfinite(amax) ? 9 - ilogbf(amax) : 0, e1 = e / 2, e2 = e - e1;
     const float f1 = ldexpf(1.f, e1), f2 = ldexpf(1.f, e2);
     if (threadIdx.x == 0) scale[m] = ldexpf(1.f, -e);
     for (int sb = warp; sb < SBp; sb += 16) {

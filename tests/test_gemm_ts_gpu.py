@@ -95,3 +95,20 @@ def test_exact_form_of_five_to_eight_rows(ctx, fmt, n, k, m):
     ctx.check_device_status()
     assert torch.equal(scaled, plain * factor)
     lin.close()
+
+
+@pytest.mark.parametrize("fmt", [ttq.FMT_Q8_0, ttq.FMT_Q6_K], ids=["q8_0", "q6_k"])
+def test_exact_form_of_rows_up_to_the_largest_bf16_value(ctx, fmt):
+    """A row whose largest magnitude is the largest finite bf16 value, 1.9921875 * 2^127: its outputs are those of the same row without
+    the power of two, times that power."""
+    n, k, m = 9500, 2048, 5
+    x = make_x(m, k, seed=9).clamp(-6, 6)
+    x[0, 77], x[3, k - 1] = 1.9921875 * 4, -1.9921875 * 4
+    factor = torch.ones(m, 1)
+    factor[0] = factor[3] = 2.0 ** 125
+    lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(make_weight(fmt, n, k, seed=8)), k)
+    plain = lin.forward(x.cuda(), out_dtype=torch.float32)
+    scaled = lin.forward((x * factor).to(torch.bfloat16).cuda(), out_dtype=torch.float32)
+    ctx.check_device_status()
+    assert plain.abs().max() < 8 and torch.equal(scaled, plain * factor.cuda())
+    lin.close()
