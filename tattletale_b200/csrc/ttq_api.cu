@@ -119,11 +119,13 @@ ttq_status alloc_weight(ttq_ctx *ctx, int fmt, int64_t N, int64_t K, ttq_weight 
     w->SBp = (K + TILE_K - 1) / TILE_K;
     w->tiled_bytes = fmt == TTQ_FMT_TQ3 ? (size_t)tq3_packed_bytes(N, K) : (size_t)w->NT * w->SBp * tile_bytes(fmt);
     w->tiles = nullptr;
-    cudaError_t e = cudaMalloc(&w->tiles, w->tiled_bytes);
+    const size_t top_at = (w->tiled_bytes + 15) & ~(size_t)15;
+    cudaError_t e = cudaMalloc(&w->tiles, top_at + (fmt == TTQ_FMT_Q8_0 || fmt == TTQ_FMT_Q6_K ? (size_t)(1 + w->NT * TILE_ROWS) * sizeof(float) : 0));
     if (e != cudaSuccess) {
         delete w;
         return cuda_fail(ctx, e, "cudaMalloc(tiled weight)");
     }
+    w->top = reinterpret_cast<float *>(w->tiles + top_at);
     if (!gemm_supported(fmt)) {
         // (the trellis format) batches beyond the decode kernels run as expansion to fp16 + plain tensor-core GEMM:
         // make sure the context's expansion scratch holds this matrix (load time; forward never allocates)
@@ -390,7 +392,7 @@ ttq_status ttq_weight_create_device(ttq_ctx *ctx, ttq_format fmt, int64_t N, int
         *out = w;
         return TTQ_OK;
     }
-    cudaError_t e = launch_repack(fmt, reinterpret_cast<const uint8_t *>(dev_blocks), w->tiles, N, K, w->NT, w->SBp,
+    cudaError_t e = launch_repack(fmt, reinterpret_cast<const uint8_t *>(dev_blocks), w->tiles, w->top, N, K, w->NT, w->SBp,
                                   (cudaStream_t)stream);
     if (e != cudaSuccess) {
         ttq_weight_destroy(w);
@@ -473,7 +475,7 @@ ttq_status ttq_weight_create(ttq_ctx *ctx, ttq_format fmt, int64_t N, int64_t K,
         cudaFree(staging);
         return s;
     }
-    e = launch_repack(fmt, staging, w->tiles, Nl, Kl, w->NT, w->SBp, ctx->host_stream);
+    e = launch_repack(fmt, staging, w->tiles, w->top, Nl, Kl, w->NT, w->SBp, ctx->host_stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->host_stream);
     cudaFree(staging);
     if (e != cudaSuccess) {
@@ -622,7 +624,7 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         (w->N + 127) / 128 * w->SBp >= 4 * (int64_t)ctx->sms) {
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
-        cudaError_t e = launch_gemm_ts_precise(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
+        cudaError_t e = launch_gemm_ts_precise(w->fmt, a, w->top, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
                                                ctx->split_counters_cap, st, &launches);
         ctx->launches += launches;
         if (e == cudaSuccess) return TTQ_OK;

@@ -24,7 +24,8 @@
 // (68.9 / 45.9 / 34.4 / 22.7); Q8_0 and Q6_K, 4096 -> 28672, 12 rows: 31.7 (69.5) and 38.3 (78.2).
 //
 // Exact form (Q8_0, Q6_K, one block of 16 rows): every weight as its fp16 rounding plus the remainder, two products into the same
-// accumulator, activations exact after a power of two per row; half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 44 us,
+// accumulator, activations exact after a power of two per row, weights beyond fp16 brought into it by a power of two
+// per weight row (ts_row_power); half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 44 us,
 // Q6_K 55 (integer decode kernel: 77 and 95); error against 64 bits as the integer kernel's or below.
 #include <cmath>
 
@@ -74,6 +75,7 @@ struct TsParams {
     const int *mt_group, *mt_row0, *n_mt;
     int64_t mt_cap;
     const float *row_scale;  // exact form: the outputs of activation row m are multiplied by row_scale[m]
+    const float *top;        // exact form: Weight::top
 };
 
 __device__ __forceinline__ void ts_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -148,9 +150,23 @@ __device__ __forceinline__ __half2 ts_as_h2(uint32_t v) { return *reinterpret_ca
 //   Q8_0  slice n = window n; run 0 = block u (chunk n), run 1 = block 4 + u (chunk 4 + n)
 //   Q6_K  slice 2 s' + n = window n of sets s' (run 0) and s' + 2 (run 1)
 
-// Writes the scale records of the tile's 16 rows (lane (r, h): half h of row r).
+// Exact form: where the weights of a matrix leave fp16 (a block's scale goes up to 65504, its weights to 128 times that in Q8_0 and 4096
+// times in Q6_K) those of every row are divided by a power of two 2^s that brings the row's largest below 2^15.  To ask costs a launch
+// up to 1 us (Q8_0, 4096 -> 28672 at 5 rows 44.5 -> 45.6, Q6_K 56.2 -> 56.2); out of line the rare case would cost nothing here but take the
+// registers that let the next linear's activation pass in beside this kernel.
+template <int FMT>
+__device__ __forceinline__ bool ts_wide(float top) { return top > (FMT == TTQ_FMT_Q8_0 ? 65504.f / 128 : 65504.f / 32); }  // `top` of Q6_K has the sub-block scale in it
+// 2^s of row n (sign 1), 2^-s (sign -1).
+template <int FMT>
+__device__ __forceinline__ float ts_row_power(const float *top, int64_t n, int sign) {
+    const float row = __ldcg(top + 1 + n);
+    const int s = ((__float_as_int(row) >> 23) & 255) - 127 + (FMT == TTQ_FMT_Q8_0 ? 7 : 5) - 14;
+    return ts_wide<FMT>(row) ? __int_as_float((127 + sign * s) << 23) : 1.f;
+}
+
+// Writes the scale records of the tile's 16 rows (lane (r, h): half h of row r).  `shrink` (exact form): 2^-s, see ts_row_power.
 template <int FMT, int MODE>
-__device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane) {
+__device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane, float shrink) {
     constexpr int TS_HDR_ROW = ts_hdr_row(FMT, MODE);
     const int r = lane & 15, h = lane >> 4;
     if constexpr (FMT == TTQ_FMT_Q4_K) {
@@ -180,14 +196,18 @@ __device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane
         sts128<16>(dst, w[4], w[5], w[6], w[7]);
     } else if constexpr (FMT == TTQ_FMT_Q8_0) {
         const uint2 hv = lds64<4096>(stage + (uint32_t)(r * 16 + h * 8));
-        sts128<0>(hdr + (uint32_t)(r * TS_HDR_ROW + h * 16), __byte_perm(hv.x, 0, 0x1010), __byte_perm(hv.x, 0, 0x3232), __byte_perm(hv.y, 0, 0x1010),
-                  __byte_perm(hv.y, 0, 0x3232));
+        uint32_t w[4] = {__byte_perm(hv.x, 0, 0x1010), __byte_perm(hv.x, 0, 0x3232), __byte_perm(hv.y, 0, 0x1010), __byte_perm(hv.y, 0, 0x3232)};
+        if (MODE == TS_PRECISE && shrink != 1.f) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = ts_h2(__hmul2(ts_as_h2(w[i]), __float2half2_rn(shrink)));
+        }
+        sts128<0>(hdr + (uint32_t)(r * TS_HDR_ROW + h * 16), w[0], w[1], w[2], w[3]);
     } else {
         // 16-wide sub-blocks 8h..8h+7: d * sc as fp16, duplicated into both halves
         const uint2 hv = lds64<3072>(stage + (uint32_t)(r * 16 + h * 8));
         uint16_t dbits;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dbits) : "r"(stage + 3328u + (uint32_t)r * 2));
-        const float d = __half2float(__ushort_as_half(dbits));
+        const float d = __half2float(__ushort_as_half(dbits)) * (MODE == TS_PRECISE ? shrink : 1.f);
         uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -452,6 +472,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             locate();
         }
     };
+    const float top = precise ? __ldcg(p.top) : 0.f;  // on its way beside the first packed tiles, first looked at with them
     if (my_count > 0) {
         // the packed weights depend on no preceding kernel: the ring fills while that one drains
         if (ts_elect()) {
@@ -498,6 +519,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(d_col + buf * nb);
             const int slot = 2 * (int)blockIdx.x + (tile == first_tile ? 0 : 1);
             float *wsp = p.ws + (size_t)slot * nb * TS_ROWS + r;
+            const float grow = precise && n < p.N && ts_wide<FMT>(top) ? ts_row_power<FMT>(p.top, n, 1) : 1.f;
             const float bias = whole && p.bias != nullptr && n < p.N ? load_as_float(p.bias, p.bias_dt, n) : 0.f;
 #pragma unroll 1
             for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -508,7 +530,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                         const int64_t at = (int64_t)(row0 + c0) * p.ldy + n;
 #pragma unroll
                         for (int i = 0; i < 16; i++)
-                            if (c0 + i < rows) store_from_float(p.y, p.y_dt, at + i * p.ldy, __uint_as_float(v[i]) * (precise ? p.row_scale[c0 + i] : 1.f) + bias);
+                            if (c0 + i < rows) store_from_float(p.y, p.y_dt, at + i * p.ldy, (precise ? __uint_as_float(v[i]) * p.row_scale[c0 + i] * grow : __uint_as_float(v[i])) + bias);
                     }
                 } else {
 #pragma unroll
@@ -551,7 +573,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             const bool have = group_of(c) * TS_GROUP_TILES + tau < p.NT;
             if (alive) alive = mbar_wait_bounded(my_bar + 8 * s, rpar, p.status);
             alive = __all_sync(0xffffffffu, alive);
-            if (have) ts_header<FMT, MODE>(stage, hdr, lane);
+            if (have) {
+                float shrink = 1.f;
+                if (precise && ts_wide<FMT>(top)) shrink = ts_row_power<FMT>(p.top, (group_of(c) * TS_GROUP_TILES + tau) * TILE_ROWS + (lane & 15), -1);
+                ts_header<FMT, MODE>(stage, hdr, lane, shrink);
+            }
             __syncwarp();  // the records are written
             // (exact form: the item takes two A stages, each two slices as rounded weights and remainders)
 #pragma unroll 1
@@ -712,6 +738,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 if (precise) o[i] *= p.row_scale[m];
+                if (precise && n + i < p.N && ts_wide<FMT>(top)) o[i] *= ts_row_power<FMT>(p.top, n + i, 1);
                 if (p.bias != nullptr && n + i < p.N) o[i] += load_as_float(p.bias, p.bias_dt, n + i);
             }
             // four outputs in one store where they lie so (y may be host memory, where every store is a transfer of its own)
@@ -806,7 +833,7 @@ cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_
     p.bias = a.bias; p.bias_dt = a.bias_dt;
     p.y = a.y; p.y_dt = a.y_dt; p.ldy = a.ldy;
     p.status = status;
-    p.row_scale = nullptr;
+    p.row_scale = nullptr; p.top = nullptr;
     p.group_tiles = nullptr; p.mt_group = nullptr; p.mt_row0 = nullptr; p.n_mt = nullptr; p.mt_cap = 0;
     cudaError_t e = launch_xh_images(a, p.Mp, Kp, xh, sms, fmt == TTQ_FMT_Q4_K ? 2 : (fmt == TTQ_FMT_Q6_K ? 3 : 4), st);
     if (e != cudaSuccess) return e;
@@ -875,7 +902,7 @@ __global__ void __launch_bounds__(512) xh_rows_kernel(const void *__restrict__ x
 
 // Q8_0 / Q6_K, up to 16 rows, with weights and activations exact: the accuracy of the integer decode kernel at the rate of
 // the tensor cores.  Not for the gated form, whose products would be rounded to fp16.
-cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
+cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *top, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                                    int64_t counters_cap, cudaStream_t st, int *launches) {
     *launches = 0;
     constexpr int NB = 16;
@@ -895,6 +922,7 @@ cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int
     p.xh = xh;
     p.ws = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + ws_at);
     p.row_scale = scale;
+    p.top = top;
     p.counters = counters;
     p.bias = a.bias; p.bias_dt = a.bias_dt;
     p.y = a.y; p.y_dt = a.y_dt; p.ldy = a.ldy;
@@ -930,7 +958,7 @@ cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int s
     p.bias = nullptr; p.bias_dt = TTQ_DT_F32;
     p.y = g.y; p.y_dt = g.y_dt; p.ldy = g.ldy;
     p.status = status;
-    p.row_scale = nullptr;
+    p.row_scale = nullptr; p.top = nullptr;
     p.group_tiles = g.group_tiles; p.mt_group = g.mt_group; p.mt_row0 = g.mt_row0; p.n_mt = g.n_mt; p.mt_cap = g.mt_cap;
     return ts_launch<TTQ_FMT_Q4_K, TS_GROUPED>(p, sms, st);
 }

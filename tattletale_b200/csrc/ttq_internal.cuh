@@ -72,6 +72,7 @@ struct Weight {
     int64_t SBp;  // 256-wide K tiles
     uint8_t *tiles;
     size_t tiled_bytes;
+    float *top;  // Q8_0, Q6_K, on the device: largest finite |scale| (d, resp. d * sc) of the matrix, then of each of 16 NT rows
 };
 
 }  // namespace ttq
@@ -259,7 +260,7 @@ struct GroupedArgs {
     unsigned *ts_counters = nullptr;
     int64_t ts_counters_cap = 0;
 };
-cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
+cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *top, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                                    int64_t counters_cap, cudaStream_t st, int *launches);
 bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms);
 cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st);
@@ -298,7 +299,7 @@ cudaError_t launch_moe_combine(const MoeRouting &r, const void *o, int o_dt, int
                                int top_k, int64_t H, void *y, int y_dt, int64_t ldy, cudaStream_t st);
 
 // launchers (defined in the .cu files); each returns the number of kernels it launched or -1
-cudaError_t launch_repack(int fmt, const uint8_t *canon, uint8_t *tiled, int64_t N, int64_t K, int64_t NT,
+cudaError_t launch_repack(int fmt, const uint8_t *canon, uint8_t *tiled, float *top, int64_t N, int64_t K, int64_t NT,
                           int64_t SBp, cudaStream_t st);
 cudaError_t launch_dequant(int fmt, const uint8_t *tiled, float *out, int64_t ld, int64_t N, int64_t K,
                            int64_t SBp, cudaStream_t st);

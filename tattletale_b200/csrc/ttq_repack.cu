@@ -111,8 +111,24 @@ __device__ uint8_t tiled_byte(const CanonTile &ct, int o) {
 }
 
 template <int FMT>
+__device__ float block_top(const CanonTile &ct, int i) {
+    // largest finite |scale| of block i of a tile: Q8_0 d of block i & 7 of row i >> 3, Q6_K d * sc of row i
+    const uint8_t *blk = FMT == TTQ_FMT_Q8_0 ? ct.block32(i >> 3, i & 7) : ct.block256(i, 210);
+    if (!blk) return 0.f;
+    const uint8_t *db = blk + (FMT == TTQ_FMT_Q8_0 ? 0 : 208);
+    float d = fabsf(__half2float(__ushort_as_half((unsigned short)(db[0] | (db[1] << 8)))));
+    if (!(d <= 65504.f)) return 0.f;
+    if (FMT == TTQ_FMT_Q6_K) {
+        int sc = 0;
+        for (int j = 0; j < 16; j++) sc = max(sc, abs((int)(int8_t)blk[192 + j]));
+        d *= (float)sc;
+    }
+    return d;
+}
+
+template <int FMT>
 __global__ void __launch_bounds__(128) repack_kernel(const uint8_t *__restrict__ canon,
-                                                     uint8_t *__restrict__ tiled, int64_t N, int64_t K,
+                                                     uint8_t *__restrict__ tiled, float *__restrict__ top, int64_t N, int64_t K,
                                                      int64_t NT, int64_t SBp) {
     constexpr int TB = tile_bytes(FMT);
     for (int64_t tile = blockIdx.x; tile < NT * SBp; tile += gridDim.x) {
@@ -123,6 +139,13 @@ __global__ void __launch_bounds__(128) repack_kernel(const uint8_t *__restrict__
 #pragma unroll
             for (int b = 0; b < 4; b++) v |= (uint32_t)tiled_byte<FMT>(ct, 4 * w + b) << (8 * b);
             dst[w] = v;
+        }
+        // (non-negative floats order like their bits; `top` is zero before the launch)
+        if (FMT != TTQ_FMT_Q4_K && threadIdx.x < (FMT == TTQ_FMT_Q8_0 ? 128 : 16)) {
+            const int bits = __float_as_int(block_top<FMT>(ct, threadIdx.x)), row = FMT == TTQ_FMT_Q8_0 ? threadIdx.x >> 3 : threadIdx.x;
+            int *words = reinterpret_cast<int *>(top);
+            if (bits > __ldcg(words)) atomicMax(words, bits);
+            atomicMax(words + 1 + ct.nt * TILE_ROWS + row, bits);
         }
     }
 }
@@ -193,12 +216,16 @@ int grid_for(int64_t work_items, int per_block, int cap) {
 
 }  // namespace
 
-cudaError_t launch_repack(int fmt, const uint8_t *canon, uint8_t *tiled, int64_t N, int64_t K, int64_t NT,
+cudaError_t launch_repack(int fmt, const uint8_t *canon, uint8_t *tiled, float *top, int64_t N, int64_t K, int64_t NT,
                           int64_t SBp, cudaStream_t st) {
+    if (fmt != TTQ_FMT_Q4_K) {
+        const cudaError_t e = cudaMemsetAsync(top, 0, (size_t)(1 + NT * TILE_ROWS) * sizeof(float), st);
+        if (e != cudaSuccess) return e;
+    }
     int grid = grid_for(NT * SBp, 1, device_sms() * 64);
-    if (fmt == TTQ_FMT_Q4_K) repack_kernel<TTQ_FMT_Q4_K><<<grid, 128, 0, st>>>(canon, tiled, N, K, NT, SBp);
-    else if (fmt == TTQ_FMT_Q8_0) repack_kernel<TTQ_FMT_Q8_0><<<grid, 128, 0, st>>>(canon, tiled, N, K, NT, SBp);
-    else repack_kernel<TTQ_FMT_Q6_K><<<grid, 128, 0, st>>>(canon, tiled, N, K, NT, SBp);
+    if (fmt == TTQ_FMT_Q4_K) repack_kernel<TTQ_FMT_Q4_K><<<grid, 128, 0, st>>>(canon, tiled, top, N, K, NT, SBp);
+    else if (fmt == TTQ_FMT_Q8_0) repack_kernel<TTQ_FMT_Q8_0><<<grid, 128, 0, st>>>(canon, tiled, top, N, K, NT, SBp);
+    else repack_kernel<TTQ_FMT_Q6_K><<<grid, 128, 0, st>>>(canon, tiled, top, N, K, NT, SBp);
     return cudaGetLastError();
 }
 

@@ -112,3 +112,32 @@ def test_exact_form_of_rows_up_to_the_largest_bf16_value(ctx, fmt):
     ctx.check_device_status()
     assert plain.abs().max() < 8 and torch.equal(scaled, plain * factor.cuda())
     lin.close()
+
+
+@pytest.mark.parametrize("top", [300.0, 1.0e4, 6.0e4])
+@pytest.mark.parametrize("fmt", [ttq.FMT_Q8_0, ttq.FMT_Q6_K], ids=["q8_0", "q6_k"])
+def test_exact_form_of_weights_beyond_fp16(ctx, fmt, top):
+    """Block scales up to `top`, so that weights leave fp16 (at 6e4 Q6_K weights reach 2^27), beside blocks of ordinary scale in the same
+    rows and in rows of their own (every third).  The weights of a row are divided by a power of two that keeps its largest below 2^15:
+    what is left out is below 2^-32 of that, so the bar of the exact form (3e-5) stands for both kinds of rows."""
+    n, k, m = 9500, 2048, 6
+    blocks = make_weight(fmt, n, k, seed=31)
+    off, size = (0, 34) if fmt == ttq.FMT_Q8_0 else (208, 210)
+    b = blocks.reshape(n, -1, size)
+    d = np.ascontiguousarray(b[..., off:off + 2]).view(np.float16)[..., 0].astype(np.float64)
+    factor = np.where(np.random.default_rng(32).random(d.shape) < 0.5, top / np.abs(d).max(), 1.0)
+    factor[::3] = 1.0
+    b[..., off:off + 2] = (d * factor).astype(np.float16)[..., None].view(np.uint8).reshape(*d.shape, 2)
+    x = make_x(m, k, seed=33)
+    lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks), k)
+    on_device = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks).cuda(), k)
+    y = lin.forward(x.cuda(), out_dtype=torch.float32)
+    same = on_device.forward(x.cuda(), out_dtype=torch.float32)
+    ctx.check_device_status()
+    want = oracle.linear(OFMT[fmt], blocks, x_bits(x), odt(torch.bfloat16), None)
+    got = y.cpu().numpy()
+    assert np.isfinite(got).all() and torch.equal(y, same)
+    assert rel_l2(got, want) < 3e-5
+    assert rel_l2(got[:, ::3], want[:, ::3]) < 3e-5
+    lin.close()
+    on_device.close()
