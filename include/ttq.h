@@ -344,8 +344,9 @@ TTQ_API ttq_status ttq_decode_attention(ttq_ctx *ctx, const void *q_dev, const v
  *     y[t] = sum_j w[t][j] * down_e( silu(gate_e x[t]) * up_e x[t] ),  e = topk_ids[t][j]
  * with E experts of identical shape, gate|up fused as one [2I][H] matrix (gate rows first) and down
  * [H][I], all Q4_K.  Router, softmax and top-k selection stay with the caller, who passes the chosen
- * expert ids and their weights.  Routing tables, the routed activation images and the intermediates
- * live in a workspace allocated by ttq_moe_create for up to max_tokens tokens; the forward call
+ * expert ids and their weights.  Routing tables, the routed activation images, the intermediates,
+ * partial sums and arrival counters live in a workspace allocated by ttq_moe_create for up to max_tokens tokens (a layer shares no
+ * scratch with other calls of its context, which may run beside it on another stream); the forward call
  * allocates nothing, copies nothing to the host and is asynchronous on `stream`.  The handle keeps
  * the experts' device pointers: destroy it before the weights. */
 TTQ_API ttq_status ttq_moe_create(ttq_ctx *ctx, int32_t n_experts, const ttq_weight *const *gate_up,

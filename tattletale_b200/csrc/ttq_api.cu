@@ -66,7 +66,20 @@ struct ttq_moe {
     MoeRouting route;
     void *ws;                      // one allocation: routing tables, activation images, intermediates
     __half *xh1, *h1, *xh2, *o2;
+    float *part;                   // tensor-memory GEMM: partial sums of row tiles that are cut over several CTAs
+    size_t part_bytes;
+    int64_t n_arrivals;            // its counters (MoeRouting::arrivals)
 };
+
+namespace {
+
+// Rows per tile of the tensor-memory GEMM by the mean number of rows per expert, up to MOE_TS_MEAN.
+constexpr int64_t MOE_TS_MEAN = 128;
+int moe_ts_rows(int64_t mean) { return mean <= 8 ? 16 : (mean <= 16 ? 32 : (mean <= 48 ? 64 : 128)); }
+// Output tiles (arrival counters) of the wider of the layer's two products.
+int64_t moe_ts_tiles(const ttq_moe *m, int64_t pairs, int BM) { return ((2 * m->I > m->H ? 2 * m->I : m->H) / 128 + 1) * (pairs / BM + m->E + 1); }
+
+}  // namespace
 
 namespace {
 
@@ -1263,7 +1276,16 @@ ttq_status ttq_moe_create(ttq_ctx *ctx, int32_t n_experts, const ttq_weight *con
     const size_t b_a = b_xh1 > b_o2 ? b_xh1 : b_o2;  // the routed input images and the routed outputs are never live together
     const size_t b_h1 = up256(sizeof(__half) * (size_t)m->rows_cap * (size_t)(2 * I));
     const size_t b_xh2 = up256(sizeof(__half) * (size_t)m->rows_cap * (size_t)(m->SBp2 * TILE_K));
-    const size_t total = 2 * b_tab + 3 * b_e + 256 + 3 * b_mt + b_rows + b_pairs + b_a + b_h1 + b_xh2;
+    // partial sums and counters of the tensor-memory GEMM, for the tallest row tiles and the most tiles that a call can have (more
+    // than SPLIT_COUNTERS tiles take the shared-memory GEMM)
+    const int64_t mean_cap = pairs / n_experts < MOE_TS_MEAN ? pairs / n_experts : MOE_TS_MEAN;
+    m->part_bytes = (size_t)2 * ctx->sms * moe_ts_rows(mean_cap) * 128 * sizeof(float);
+    for (int64_t mean : {(int64_t)8, (int64_t)16, (int64_t)48, MOE_TS_MEAN}) {
+        const int64_t most = (mean + 1) * n_experts - 1, tiles = moe_ts_tiles(m, most < pairs ? most : pairs, moe_ts_rows(mean));
+        if (tiles > m->n_arrivals) m->n_arrivals = tiles < SPLIT_COUNTERS ? tiles : SPLIT_COUNTERS;
+    }
+    const size_t b_arr = up256(sizeof(unsigned) * (size_t)m->n_arrivals);
+    const size_t total = 2 * b_tab + b_arr + 3 * b_e + 256 + 3 * b_mt + b_rows + b_pairs + b_a + b_h1 + b_xh2 + m->part_bytes;
     cudaError_t e = cudaMalloc(&m->ws, total);
     if (e != cudaSuccess) {
         delete m;
@@ -1272,6 +1294,7 @@ ttq_status ttq_moe_create(ttq_ctx *ctx, int32_t n_experts, const ttq_weight *con
     uint8_t *q = reinterpret_cast<uint8_t *>(m->ws);
     m->d_gate_up = reinterpret_cast<const uint8_t **>(q); q += b_tab;
     m->d_down = reinterpret_cast<const uint8_t **>(q); q += b_tab;
+    m->route.arrivals = reinterpret_cast<unsigned *>(q); q += b_arr;
     m->route.counts = reinterpret_cast<int *>(q); q += b_e;
     m->route.row_start = reinterpret_cast<int *>(q); q += b_e;
     m->route.cursor = reinterpret_cast<int *>(q); q += b_e;
@@ -1283,7 +1306,8 @@ ttq_status ttq_moe_create(ttq_ctx *ctx, int32_t n_experts, const ttq_weight *con
     m->route.slot_of = reinterpret_cast<int *>(q); q += b_pairs;
     m->xh1 = reinterpret_cast<__half *>(q); m->o2 = m->xh1; q += b_a;
     m->h1 = reinterpret_cast<__half *>(q); q += b_h1;
-    m->xh2 = reinterpret_cast<__half *>(q);
+    m->xh2 = reinterpret_cast<__half *>(q); q += b_xh2;
+    m->part = reinterpret_cast<float *>(q);
     std::vector<const uint8_t *> tab((size_t)2 * n_experts);
     for (int x = 0; x < n_experts; x++) {
         tab[x] = gate_up[x]->tiles;
@@ -1331,8 +1355,8 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
     // per expert; above, 256-row tiles of the shared-memory GEMM expand a weight once for more rows.
     // Measured, whole layer, us (shared-memory GEMM in brackets): 128 experts of 2048 x 768, top 8: 24 tokens 140 (249), 200 194
     // (339), 700 261 (402), 1500 422 (485); 8 experts of 4096 x 1536, top 2: 64 tokens 75 (138), 500 125 (166).
-    bool ts = mean <= 128;
-    if (ts) BM = mean <= 8 ? 16 : (mean <= 16 ? 32 : (mean <= 48 ? 64 : 128));
+    bool ts = mean <= MOE_TS_MEAN;
+    if (ts) BM = moe_ts_rows(mean);
     static const int force_bm = []() {
         const char *v = getenv("TTQ_MOE_BM");
         return v ? atoi(v) : 0;
@@ -1342,8 +1366,7 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
         ts = false;
     }
     if (ts) {
-        const int64_t groups = (2 * m->I > m->H ? 2 * m->I : m->H) / 128 + 1;
-        ts = groups * (pairs / BM + m->E + 1) <= ctx->split_counters_cap;
+        ts = moe_ts_tiles(m, pairs, BM) <= m->n_arrivals;
         if (!ts) BM = mean <= 64 ? 64 : 128;
     }
     const int64_t unit = BM == 384 ? 128 : BM;
@@ -1364,10 +1387,10 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
     g.mt_row0 = m->route.mt_row0; g.mt_mh = m->route.mt_mh; g.rows_total = m->route.n_mt + 1; g.mt_cap = mt_cap;
     g.y = m->h1; g.y_dt = TTQ_DT_F16; g.ldy = 2 * m->I;
     if (ts) {
-        g.ts_ws = reinterpret_cast<float *>(ctx->xh);  // (the context's image scratch: 2 x SMs x 128 rows x 128 floats are 19 of its 64 MB)
-        g.ts_ws_bytes = (size_t)ctx->xh_capacity * sizeof(__half);
-        g.ts_counters = ctx->split_counters;
-        g.ts_counters_cap = ctx->split_counters_cap;
+        g.ts_ws = m->part;
+        g.ts_ws_bytes = m->part_bytes;
+        g.ts_counters = m->route.arrivals;
+        g.ts_counters_cap = m->n_arrivals;
     }
     e = launch_gemm_grouped(g, m->xh1, ctx->sms, ctx->dev_status, st, &n);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "grouped gate|up launch");

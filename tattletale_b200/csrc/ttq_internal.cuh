@@ -287,6 +287,7 @@ cudaError_t launch_decode_attention(const void *q, const void *k_cache, const vo
 
 // Routing and combination of a mixture-of-experts layer (ttq_moe.cu).
 struct MoeRouting {
+    unsigned *arrivals;                // [n_arrivals] counters of the grouped GEMM; they and the counts behind them are cleared per call
     int *counts, *row_start, *cursor;  // [E]
     int *n_mt;                         // [1] row tiles in use; [1] routed rows in use
     int *mt_group, *mt_row0, *mt_mh;   // [Mp / 64] each

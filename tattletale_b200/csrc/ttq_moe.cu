@@ -131,7 +131,8 @@ cudaError_t launch_moe_route(const MoeRouting &r, const int *topk_ids, int64_t T
                              int64_t mt_cap, cudaStream_t st, int *launches) {
     *launches = 0;
     const int64_t pairs = T * top_k;
-    cudaError_t e = cudaMemsetAsync(r.counts, 0, sizeof(int) * (size_t)E, st);
+    // (the arrival counters in front of the counts too: a call that gave up a wait may have left some behind)
+    cudaError_t e = cudaMemsetAsync(r.arrivals, 0, (size_t)(reinterpret_cast<uint8_t *>(r.counts + E) - reinterpret_cast<uint8_t *>(r.arrivals)), st);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(r.row_src, 0xff, sizeof(int) * (size_t)Mp, st);  // every row is padding until a pair claims it
     if (e != cudaSuccess) return e;

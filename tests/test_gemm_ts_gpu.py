@@ -141,3 +141,40 @@ def test_exact_form_of_weights_beyond_fp16(ctx, fmt, top):
     assert rel_l2(got[:, ::3], want[:, ::3]) < 3e-5
     lin.close()
     on_device.close()
+
+
+def run_on_two_streams(ctx, first, second, rounds=20):
+    """Both calls' results in turn, then enqueued side by side: every round must give the same bits."""
+    want = first().clone(), second().clone()
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(rounds):
+        got = []
+        for stream, call in zip(streams, (first, second)):
+            with torch.cuda.stream(stream):
+                got.append([call() for _ in range(4)])
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for ys, w in zip(got, want) for y in ys)
+    ctx.check_device_status()
+
+
+@pytest.mark.parametrize("beside", ["linear", "layer"])
+def test_expert_layer_beside_another_call(ctx, beside):
+    """An expert layer keeps its partial sums and arrival counters to itself: a linear of the same context or a second layer may run
+    on another stream at the same time."""
+    from test_moe_gpu import build, routing
+
+    hidden, inter, n_exp, top_k, t = 1024, 768, 32, 4, 24
+    ids, w = (torch.from_numpy(v).cuda() for v in routing(t, n_exp, top_k, seed=3))
+    x = make_x(t, hidden, 5).cuda()
+    layer = build(ctx, n_exp, hidden, inter, top_k, max_tokens=64, seed=41)[0]
+    if beside == "layer":
+        other = build(ctx, n_exp, hidden, inter, top_k, max_tokens=64, seed=42)[0]
+        call = lambda: other.forward(x, ids, w)
+    else:
+        other = ttq.QuantLinear(ctx, ttq.FMT_Q4_K, torch.from_numpy(make_weight(ttq.FMT_Q4_K, 2048, 4096, seed=43)), 4096)
+        rows = make_x(64, 4096, 6).cuda()
+        call = lambda: other.forward(rows)
+    run_on_two_streams(ctx, lambda: layer.forward(x, ids, w), call)
+    layer.close()
+    other.close()
