@@ -40,6 +40,7 @@ struct ttq_ctx {
     size_t split_ws_bytes;
     unsigned *split_counters;   // their per-row-tile arrival counters, zero between launches
     int64_t split_counters_cap;
+    unsigned *ts_counters;      // arrival counters of the tensor-memory GEMM (SPLIT_COUNTERS of them, zero between launches)
     // device staging for the *_host entry points
     uint8_t *stage_x, *stage_y, *stage_b;
     size_t stage_x_bytes, stage_y_bytes, stage_b_bytes;
@@ -335,6 +336,8 @@ ttq_status ttq_init(int device, ttq_ctx **out) {
     if (e == cudaSuccess) e = cudaMalloc(&ctx->split_ws, SPLIT_WS_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->split_counters, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->split_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->ts_counters, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(ctx->ts_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_x, STAGE_X_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_y, STAGE_Y_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_b, STAGE_B_BYTES);
@@ -377,6 +380,7 @@ ttq_status ttq_destroy(ttq_ctx *ctx) {
     cudaFree(ctx->xh);
     cudaFree(ctx->split_ws);
     cudaFree(ctx->split_counters);
+    cudaFree(ctx->ts_counters);
     cudaFree(ctx->wimg);
     cudaFree(ctx->tq_x1);
     cudaFree(ctx->tq_y1);
@@ -618,8 +622,8 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         const int64_t groups = (w->N + 127) / 128;
         const bool large = groups * w->SBp >= 5 * (int64_t)ctx->sms || w->SBp >= 32;
         if (M <= 192 || (M <= 256 && large && groups <= ctx->sms)) {
-            cudaError_t e = launch_gemm_ts(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
-                                           ctx->split_counters_cap, st, &launches);
+            cudaError_t e = launch_gemm_ts(w->fmt, a, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->ts_counters, SPLIT_COUNTERS,
+                                           st, &launches);
             ctx->launches += launches;
             if (e == cudaSuccess) return TTQ_OK;
             if (e != cudaErrorNotSupported) return cuda_fail(ctx, e, "linear forward (tensor-memory GEMM) launch");
@@ -688,6 +692,12 @@ void *host_mapping(ttq_ctx *ctx, const void *p) {
     return at.devicePointer;
 }
 
+// A kernel that gave up a wait may have left arrival counters behind.
+void clear_counters(ttq_ctx *ctx, cudaStream_t st) {
+    cudaMemsetAsync(ctx->split_counters, 0, (size_t)ctx->split_counters_cap * sizeof(unsigned), st);
+    cudaMemsetAsync(ctx->ts_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned), st);
+}
+
 // Waits for the context's host stream; a kernel that gave up a bounded wait has raised the mapped host flag by then.
 ttq_status host_stream_sync(ttq_ctx *ctx) {
     cudaStream_t st = ctx->host_stream;
@@ -698,7 +708,7 @@ ttq_status host_stream_sync(ttq_ctx *ctx) {
         TTQ_CUDA(ctx, cudaStreamSynchronize(st));
         const int seen = ctx->host_status[1];
         cudaMemsetAsync(ctx->dev_status, 0, sizeof(int), st);
-        cudaMemsetAsync(ctx->split_counters, 0, (size_t)ctx->split_counters_cap * sizeof(unsigned), st);
+        clear_counters(ctx, st);
         return fail(ctx, TTQ_ERR_TIMEOUT, "a kernel gave up a bounded wait (status word 0x%x); results of that call are invalid", seen);
     }
     return TTQ_OK;
@@ -1064,8 +1074,7 @@ ttq_status ttq_device_status(ttq_ctx *ctx, void *stream) {
     if (host != 0) {
         ctx->host_status[0] = 0;
         cudaMemsetAsync(ctx->dev_status, 0, sizeof(int), (cudaStream_t)stream);
-        // a kernel that gave up may have left K-split arrival counters behind
-        cudaMemsetAsync(ctx->split_counters, 0, (size_t)ctx->split_counters_cap * sizeof(unsigned), (cudaStream_t)stream);
+        clear_counters(ctx, (cudaStream_t)stream);
         return fail(ctx, TTQ_ERR_TIMEOUT, "a kernel gave up a bounded wait (status word 0x%x); results of that call are invalid", host);
     }
     return TTQ_OK;

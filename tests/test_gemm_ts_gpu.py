@@ -178,3 +178,14 @@ def test_expert_layer_beside_another_call(ctx, beside):
     run_on_two_streams(ctx, lambda: layer.forward(x, ids, w), call)
     layer.close()
     other.close()
+
+
+def test_prefill_rows_beside_decode_rows(ctx):
+    """Q4_K at 64 rows (the tensor-memory kernel) and at 8 rows of a long K (the one-launch kernel, K cut over CTAs) on two streams: each
+    counts the arrivals of its pieces on counters of its own."""
+    big = ttq.QuantLinear(ctx, ttq.FMT_Q4_K, torch.from_numpy(make_weight(ttq.FMT_Q4_K, 2048, 4096, seed=51)), 4096)
+    long = ttq.QuantLinear(ctx, ttq.FMT_Q4_K, torch.from_numpy(make_weight(ttq.FMT_Q4_K, 1024, 14336, seed=52)), 14336)
+    x64, x8 = make_x(64, 4096, 53).cuda(), make_x(8, 14336, 54).cuda()
+    run_on_two_streams(ctx, lambda: big.forward(x64), lambda: long.forward(x8))
+    big.close()
+    long.close()
