@@ -18,6 +18,12 @@
  *    device, as in the reference's single-threaded model.
  *  - The caller owns x, y, bias and the stream.  The library owns repacked weights and its scratch.
  *  - `stream` is a cudaStream_t passed as void* (NULL = the legacy default stream).
+ *  - Calls of one context share its scratch: on one stream they may follow each other in any order.  Calls that may overlap
+ *    on the GPU (two streams; the host entry points run on the context's own) must not be of the same kind:
+ *      a  Q4_K up to 2 rows, Q8_0 / Q6_K up to 8, ttq_add_rmsnorm_prepare and ttq_linear_forward_prepared
+ *      b  Q4_K of 3 to 16 rows (2 where K >= 8192); ttq_linear_forward_allreduce is of kinds a and b
+ *      c  Q4_K from 17 rows, Q8_0 / Q6_K from 9, trellis from 65        d  every trellis call        e  ttq_decode_attention
+ *    An expert layer (ttq_moe) has a workspace of its own and overlaps with anything but itself.
  *  - Device-pointer entry points are asynchronous on `stream`; *_host entry points copy in, run,
  *    copy out and synchronise before returning.
  *  - Shapes: W is [N = out_features][K = in_features]; x is [M][ldx] (ldx >= K, in elements);

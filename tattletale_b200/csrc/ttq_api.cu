@@ -40,7 +40,10 @@ struct ttq_ctx {
     size_t split_ws_bytes;
     unsigned *split_counters;   // their per-row-tile arrival counters, zero between launches
     int64_t split_counters_cap;
-    unsigned *ts_counters;      // arrival counters of the tensor-memory GEMM (SPLIT_COUNTERS of them, zero between launches)
+    unsigned *ts_counters;      // arrival counters of the tensor-memory GEMM, then those of its exact form (SPLIT_COUNTERS each, zero
+                                //   between launches)
+    __half *exact;              // the exact form's images, row scales and partial sums (fixed at init)
+    int64_t exact_capacity;     // in halves
     // device staging for the *_host entry points
     uint8_t *stage_x, *stage_y, *stage_b;
     size_t stage_x_bytes, stage_y_bytes, stage_b_bytes;
@@ -336,8 +339,10 @@ ttq_status ttq_init(int device, ttq_ctx **out) {
     if (e == cudaSuccess) e = cudaMalloc(&ctx->split_ws, SPLIT_WS_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->split_counters, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->split_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->ts_counters, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(ctx->ts_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->ts_counters, (size_t)2 * SPLIT_COUNTERS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(ctx->ts_counters, 0, (size_t)2 * SPLIT_COUNTERS * sizeof(unsigned));
+    ctx->exact_capacity = gemm_ts_precise_halves(XQ_CAPACITY_K, ctx->sms);
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->exact, (size_t)ctx->exact_capacity * sizeof(__half));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_x, STAGE_X_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_y, STAGE_Y_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->stage_b, STAGE_B_BYTES);
@@ -381,6 +386,7 @@ ttq_status ttq_destroy(ttq_ctx *ctx) {
     cudaFree(ctx->split_ws);
     cudaFree(ctx->split_counters);
     cudaFree(ctx->ts_counters);
+    cudaFree(ctx->exact);
     cudaFree(ctx->wimg);
     cudaFree(ctx->tq_x1);
     cudaFree(ctx->tq_y1);
@@ -641,8 +647,8 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
         (w->N + 127) / 128 * w->SBp >= 4 * (int64_t)ctx->sms) {
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
-        cudaError_t e = launch_gemm_ts_precise(w->fmt, a, w->top, ctx->xh, ctx->xh_capacity, ctx->sms, ctx->dev_status, ctx->split_counters,
-                                               ctx->split_counters_cap, st, &launches);
+        cudaError_t e = launch_gemm_ts_precise(w->fmt, a, w->top, ctx->exact, ctx->exact_capacity, ctx->sms, ctx->dev_status,
+                                               ctx->ts_counters + SPLIT_COUNTERS, SPLIT_COUNTERS, st, &launches);
         ctx->launches += launches;
         if (e == cudaSuccess) return TTQ_OK;
         if (e != cudaErrorNotSupported) return cuda_fail(ctx, e, "linear forward (tensor-memory decode) launch");
@@ -695,7 +701,7 @@ void *host_mapping(ttq_ctx *ctx, const void *p) {
 // A kernel that gave up a wait may have left arrival counters behind.
 void clear_counters(ttq_ctx *ctx, cudaStream_t st) {
     cudaMemsetAsync(ctx->split_counters, 0, (size_t)ctx->split_counters_cap * sizeof(unsigned), st);
-    cudaMemsetAsync(ctx->ts_counters, 0, (size_t)SPLIT_COUNTERS * sizeof(unsigned), st);
+    cudaMemsetAsync(ctx->ts_counters, 0, (size_t)2 * SPLIT_COUNTERS * sizeof(unsigned), st);
 }
 
 // Waits for the context's host stream; a kernel that gave up a bounded wait has raised the mapped host flag by then.

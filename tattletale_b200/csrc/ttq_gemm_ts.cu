@@ -900,12 +900,17 @@ __global__ void __launch_bounds__(512) xh_rows_kernel(const void *__restrict__ x
 
 }  // namespace
 
+constexpr int TS_PRECISE_ROWS = 16;
+int64_t gemm_ts_precise_halves(int64_t Kp, int sms) {
+    return TS_PRECISE_ROWS * Kp + (256 + (int64_t)2 * sms * TS_PRECISE_ROWS * TS_ROWS * (int64_t)sizeof(float)) / (int64_t)sizeof(__half);
+}
+
 // Q8_0 / Q6_K, up to 16 rows, with weights and activations exact: the accuracy of the integer decode kernel at the rate of
 // the tensor cores.  Not for the gated form, whose products would be rounded to fp16.
 cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *top, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                                    int64_t counters_cap, cudaStream_t st, int *launches) {
     *launches = 0;
-    constexpr int NB = 16;
+    constexpr int NB = TS_PRECISE_ROWS;
     if ((fmt != TTQ_FMT_Q8_0 && fmt != TTQ_FMT_Q6_K) || a.M < 1 || a.M > NB || a.gated) return cudaErrorNotSupported;
     TsParams p;
     p.mbs = 1; p.nb = NB;
@@ -917,7 +922,7 @@ cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *to
     const int grid = ts_grid(p.T, groups, p.SBp, NB, sms);
     const int64_t Kp = a.SBp * TILE_K;
     const size_t xh_bytes = (size_t)NB * Kp * sizeof(__half), ws_at = xh_bytes + 256;  // 256: the row scales
-    if (ws_at + (size_t)2 * grid * NB * TS_ROWS * sizeof(float) > (size_t)xh_capacity * sizeof(__half) || groups > counters_cap) return cudaErrorNotSupported;
+    if (gemm_ts_precise_halves(Kp, grid) > xh_capacity || groups > counters_cap) return cudaErrorNotSupported;
     float *scale = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + xh_bytes);
     p.xh = xh;
     p.ws = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + ws_at);

@@ -262,6 +262,7 @@ struct GroupedArgs {
 };
 cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *top, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                                    int64_t counters_cap, cudaStream_t st, int *launches);
+int64_t gemm_ts_precise_halves(int64_t Kp, int sms);  // scratch of the exact form, in halves
 bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms);
 cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st);
 cudaError_t launch_gemm_grouped(const GroupedArgs &g, __half *xh, int sms, int *status, cudaStream_t st, int *launches);

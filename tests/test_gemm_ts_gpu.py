@@ -189,3 +189,27 @@ def test_prefill_rows_beside_decode_rows(ctx):
     run_on_two_streams(ctx, lambda: big.forward(x64), lambda: long.forward(x8))
     big.close()
     long.close()
+
+
+def test_exact_rows_of_a_host_batch_beside_a_prefill(ctx):
+    """Q8_0 at six rows in a recorded batch, which runs on the context's own stream, while a 64-row linear is in flight on the caller's: the
+    exact form has its own images, partial sums and counters."""
+    n, k = 9500, 2048
+    small = ttq.QuantLinear(ctx, ttq.FMT_Q8_0, torch.from_numpy(make_weight(ttq.FMT_Q8_0, n, k, seed=61)), k)
+    big = ttq.QuantLinear(ctx, ttq.FMT_Q4_K, torch.from_numpy(make_weight(ttq.FMT_Q4_K, 4096, 4096, seed=62)), 4096)
+    x6, x64 = make_x(6, k, 63).pin_memory(), make_x(64, 4096, 64).cuda()
+    y6 = torch.zeros(6, n, dtype=torch.bfloat16).pin_memory()
+    batch = ttq.HostBatch(ctx, [(small, x6, y6)])
+    batch.run()
+    want6, want64 = y6.clone(), big.forward(x64)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        y6.zero_()
+        ys = [big.forward(x64) for _ in range(8)]
+        batch.run()
+        torch.cuda.synchronize()
+        assert torch.equal(y6, want6) and all(torch.equal(y, want64) for y in ys)
+    ctx.check_device_status()
+    batch.close()
+    small.close()
+    big.close()
