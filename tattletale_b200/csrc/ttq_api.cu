@@ -1389,7 +1389,7 @@ ttq_status ttq_moe_forward(ttq_ctx *ctx, ttq_moe *m, const void *x_dev, ttq_dtyp
     if (Mp > m->rows_cap) Mp = m->rows_cap / unit * unit;
     const int64_t mt_cap = BM == 384 ? pairs / 384 + m->E + 1 : Mp / BM;
     int n = 0;
-    cudaError_t e = launch_moe_route(m->route, topk_ids_dev, T, m->top_k, m->E, BM, Mp, mt_cap, st, &n);
+    cudaError_t e = launch_moe_route(m->route, topk_ids_dev, T, m->top_k, m->E, BM, Mp, mt_cap, ts, st, &n);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "routing launch");
     ctx->launches += n;
     GroupedArgs g;

@@ -296,7 +296,7 @@ struct MoeRouting {
     int *slot_of;                      // [T * top_k]
 };
 cudaError_t launch_moe_route(const MoeRouting &r, const int *topk_ids, int64_t T, int top_k, int E, int BM, int64_t Mp,
-                             int64_t mt_cap, cudaStream_t st, int *launches);
+                             int64_t mt_cap, bool ordered, cudaStream_t st, int *launches);
 cudaError_t launch_moe_combine(const MoeRouting &r, const void *o, int o_dt, int64_t ldo, const float *topk_w, int64_t T,
                                int top_k, int64_t H, void *y, int y_dt, int64_t ldy, cudaStream_t st);
 

@@ -7,9 +7,13 @@
 //
 //   route_count   histogram of the expert ids
 //   route_plan    prefix over the experts -> first row of each expert, expert of each row tile, tile count
-//   route_scatter slot of every pair (atomic cursor per expert), source token of every slot
-//   combine       y[t] = sum_j w[t][j] * o[slot(t, j)]   (fixed order over j: the result does not depend
-//                 on the order in which the atomics handed out the slots)
+//   route_scatter slot of every pair (atomic cursor per expert), source token of every slot; `ordered` for the tensor-memory
+//                 GEMM: slots in the order of the pairs
+//   combine       y[t] = sum_j w[t][j] * o[slot(t, j)]   (fixed order over j)
+//
+// The result does not depend on the order in which the atomics handed out the slots: the shared-memory GEMM adds up every row in
+// the same order wherever it lies.  The tensor-memory GEMM cuts each row tile along K at places of its own, so there a row's tile
+// has to be the same in every call.
 //
 // The reference has no mixture-of-experts layer; the dataflow is the gated MLP of
 // workspace/transformers/src/layers/mlp.nim:56-60 applied per expert, weighted and summed.
@@ -84,6 +88,50 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int *__restric
     }
 }
 
+// One block per expert: its pairs in ascending order, 1024 of all pairs a step.  (1500 tokens of 8 choices among 128 experts: 12 steps;
+// a call with more rows per expert than the tensor-memory GEMM serves keeps the atomics.)
+__global__ void __launch_bounds__(256) route_scatter_ordered_kernel(const int *__restrict__ ids, int64_t pairs, int top_k, int E, int64_t Mp,
+                                                                    const int *__restrict__ row_start, int *__restrict__ slot_of,
+                                                                    int *__restrict__ row_src) {
+    __shared__ int warp_count[8];
+    const int e = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int base = row_start[e];
+    for (int64_t i0 = 0; i0 < pairs; i0 += 1024) {
+        const int64_t i = i0 + 4 * threadIdx.x;
+        int id[4], count = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            id[q] = i + q < pairs ? ids[i + q] : -1;
+            count += id[q] == e ? 1 : 0;
+            if (e == 0 && i + q < pairs && (id[q] < 0 || id[q] >= E)) slot_of[i + q] = -1;
+        }
+        int upto = count;  // of the warp's threads up to this one
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        if (lane == 31) warp_count[warp] = upto;
+        __syncthreads();
+        int before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            before += w < warp ? warp_count[w] : 0;
+            total += warp_count[w];
+        }
+        int slot = base + before + upto - count;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (id[q] != e) continue;
+            if (slot < Mp) row_src[slot] = (int)((i + q) / top_k);
+            slot_of[i + q] = slot < Mp ? slot : -1;
+            slot++;
+        }
+        base += total;
+        __syncthreads();
+    }
+}
+
 // 8 outputs per thread; o rows are fp16 or bf16 (16-byte aligned rows take the vector path)
 __global__ void __launch_bounds__(256) combine_kernel(const void *__restrict__ o, int o_dt, int64_t ldo, const int *__restrict__ slot_of,
                                                       const float *__restrict__ w, int64_t T, int top_k, int64_t H, void *__restrict__ y,
@@ -128,7 +176,7 @@ unsigned grid_of(int64_t items, int cap) {
 }  // namespace
 
 cudaError_t launch_moe_route(const MoeRouting &r, const int *topk_ids, int64_t T, int top_k, int E, int BM, int64_t Mp,
-                             int64_t mt_cap, cudaStream_t st, int *launches) {
+                             int64_t mt_cap, bool ordered, cudaStream_t st, int *launches) {
     *launches = 0;
     const int64_t pairs = T * top_k;
     // (the arrival counters in front of the counts too: a call that gave up a wait may have left some behind)
@@ -139,8 +187,11 @@ cudaError_t launch_moe_route(const MoeRouting &r, const int *topk_ids, int64_t T
     route_count_kernel<<<grid_of(pairs, device_sms() * 4), 256, 0, st>>>(topk_ids, pairs, E, r.counts);
     route_plan_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)(E + 1), st>>>(r.counts, E, BM, (int)mt_cap, r.row_start, r.cursor, r.mt_group,
                                                                           r.mt_row0, r.mt_mh, r.n_mt);
-    route_scatter_kernel<<<grid_of(pairs, device_sms() * 4), 256, 0, st>>>(topk_ids, pairs, top_k, E, Mp, r.row_start, r.cursor, r.slot_of,
-                                                                  r.row_src);
+    if (ordered)
+        route_scatter_ordered_kernel<<<E, 256, 0, st>>>(topk_ids, pairs, top_k, E, Mp, r.row_start, r.slot_of, r.row_src);
+    else
+        route_scatter_kernel<<<grid_of(pairs, device_sms() * 4), 256, 0, st>>>(topk_ids, pairs, top_k, E, Mp, r.row_start, r.cursor, r.slot_of,
+                                                                               r.row_src);
     *launches = 3;
     return cudaGetLastError();
 }

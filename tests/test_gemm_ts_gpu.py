@@ -213,3 +213,20 @@ def test_exact_rows_of_a_host_batch_beside_a_prefill(ctx):
     batch.close()
     small.close()
     big.close()
+
+
+@pytest.mark.parametrize("t,n_exp,top_k", [(250, 8, 4), (600, 64, 8), (1100, 16, 1)])
+def test_expert_layer_repeats_itself(ctx, t, n_exp, top_k):
+    """Experts with more rows than a tile: a row lies in the same tile in every call, so its sum has the same order and the same bits."""
+    from test_moe_gpu import build, routing
+
+    hidden, inter = 1024, 768
+    layer = build(ctx, n_exp, hidden, inter, top_k, max_tokens=t, seed=71)[0]
+    ids, w = (torch.from_numpy(v).cuda() for v in routing(t, n_exp, top_k, seed=72, skew=True))
+    ids[5, 0] = -1
+    x = make_x(t, hidden, 73).cuda()
+    first = layer.forward(x, ids, w, out=torch.empty(t, hidden, device="cuda"))
+    for _ in range(20):
+        assert torch.equal(layer.forward(x, ids, w, out=torch.empty(t, hidden, device="cuda")), first)
+    ctx.check_device_status()
+    layer.close()
