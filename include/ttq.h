@@ -293,6 +293,11 @@ TTQ_API ttq_status ttq_linear_forward_gated(ttq_ctx *ctx, const ttq_weight *w, c
                                             int64_t M, int64_t ld_gate_up, const void *bias_dev, ttq_dtype bias_dt,
                                             void *y_dev, ttq_dtype y_dt, int64_t ldy, void *stream);
 
+/* 1 where ttq_linear_forward_gated is the faster way to a gated MLP's down projection of M rows, 0 where ttq_silu_and_mul
+ * and ttq_linear_forward are (the only way for TTQ_FMT_TQ3).  A few rows of Q4_K run a kernel whose every CTA converts the
+ * activations for itself; with silu(gate) * up in that conversion, long rows cost more than the launch it saves. */
+TTQ_API int32_t ttq_linear_gated_pays(const ttq_ctx *ctx, const ttq_weight *w, int64_t M);
+
 /* ---- adjacent step: silu_and_mul (kernels/activations.nim:14-38) ---------------------------- */
 
 /* out[m][h] = silu(in[m][h]) * in[m][H + h]; in is [M][ld_in] with 2H used columns, out [M][ld_out].

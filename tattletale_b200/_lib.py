@@ -59,6 +59,7 @@ SIGNATURES = {
     "ttq_host_batch_destroy": (_ci, [_vp]),
     "ttq_linear_forward_static": (_ci, [_vp, _vp, _ci, _i64, _i64, _vp, _ci, _vp, _ci, _i64, _vp, ctypes.c_char_p, _sz]),
     "ttq_static_status": (_ci, [_vp, ctypes.c_char_p, _sz]),
+    "ttq_linear_gated_pays": (_ci, [_vp, _vp, _i64]),
     "ttq_linear_forward_gated": (_ci, [_vp, _vp, _vp, _ci, _i64, _i64, _vp, _ci, _vp, _ci, _i64, _vp]),
     "ttq_comm_create": (_ci, [_vp, _ci, _ci, _i64, _ci, _pp, _vp]),
     "ttq_comm_connect": (_ci, [_vp, _vp]),

@@ -540,6 +540,13 @@ ttq_status ttq_dequantize(ttq_ctx *ctx, const ttq_weight *w, float *dev_out, int
     return TTQ_OK;
 }
 
+// Rows that ttq_linear_forward gives to the one-launch Q4_K kernel.
+static bool q4k_one_launch(const ttq_weight *w, int64_t M) {
+    static const bool use_mma = env_flag("TTQ_Q4K_MMA", true);
+    constexpr int64_t MMA_MIN_M = 3, MMA_MAX_M = 16;
+    return w->fmt == TTQ_FMT_Q4_K && use_mma && (M >= MMA_MIN_M || (M == 2 && w->SBp >= 32)) && M <= MMA_MAX_M;
+}
+
 static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const void *x_dev, ttq_dtype x_dt, int64_t M,
                               int64_t ldx, const void *bias_dev, ttq_dtype bias_dt, void *y_dev, ttq_dtype y_dt,
                               int64_t ldy, void *stream, bool gated) {
@@ -593,11 +600,9 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
     // Q4_K batches of 3 to 16 rows: one kernel (fp16 tensor-core instructions on exact integer operands, activations
     // converted inside the kernel).  Up to 2 rows the integer decode kernel below is faster, beyond 16 the tcgen05 path.
     // TTQ_Q4K_MMA=0 switches the kernel off.
-    static const bool use_mma = env_flag("TTQ_Q4K_MMA", true);
     // (two rows of a long K -- 8192 and more -- also go there: their planes leave room for one small CTA per SM only in
     // the integer kernel; measured 17.3 against 21.1 us on 14336 -> 4096)
-    constexpr int64_t MMA_MIN_M = 3, MMA_MAX_M = 16;
-    if (w->fmt == TTQ_FMT_Q4_K && use_mma && (M >= MMA_MIN_M || (M == 2 && w->SBp >= 32)) && M <= MMA_MAX_M) {
+    if (q4k_one_launch(w, M)) {
         a.x = x_dev; a.M = M; a.y = y_dev;
         int launches = 0;
         cudaError_t e = launch_q4k_mma(a, ctx->sms, ctx->dev_status, ctx->trace, ctx->split_ws, ctx->split_ws_bytes, ctx->split_counters,
@@ -670,6 +675,14 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
 ttq_status ttq_linear_forward(ttq_ctx *ctx, const ttq_weight *w, const void *x_dev, ttq_dtype x_dt, int64_t M, int64_t ldx,
                               const void *bias_dev, ttq_dtype bias_dt, void *y_dev, ttq_dtype y_dt, int64_t ldy, void *stream) {
     return linear_forward_impl(ctx, w, x_dev, x_dt, M, ldx, bias_dev, bias_dt, y_dev, y_dt, ldy, stream, false);
+}
+
+int32_t ttq_linear_gated_pays(const ttq_ctx *ctx, const ttq_weight *w, int64_t M) {
+    if (!ctx || !w || w->fmt == TTQ_FMT_TQ3) return 0;
+    if (!q4k_one_launch(w, M)) return 1;
+    LinearArgs a = {};
+    a.N = w->N; a.K = w->K; a.NT = w->NT; a.SBp = w->SBp; a.M = M;
+    return q4k_mma_gated_pays(a, ctx->sms, ctx->split_ws_bytes, ctx->split_counters_cap) ? 1 : 0;
 }
 
 ttq_status ttq_linear_forward_gated(ttq_ctx *ctx, const ttq_weight *w, const void *gate_up_dev, ttq_dtype x_dt, int64_t M,

@@ -323,6 +323,8 @@ cudaError_t launch_q4k_umma(const LinearArgs &a, const XqView &xq, int64_t xq_ca
 // (ttq_q4k_mma.cu).  `ws` / `counters`: fp32 workspace and per-row-tile arrival counters (zero between launches)
 // for matrices whose K is split across CTAs.  cudaErrorNotSupported: the caller takes another path.
 bool q4k_mma_supported(const LinearArgs &a);
+// whether the gated form is faster on this kernel than a separate activation pass and the plain form
+bool q4k_mma_gated_pays(const LinearArgs &a, int sms, size_t ws_bytes, int64_t counters_cap);
 cudaError_t launch_q4k_mma(const LinearArgs &a, int sms, int *status, unsigned long long *trace, float *ws, size_t ws_bytes,
                            unsigned *counters, int64_t counters_cap, cudaStream_t st, int *launches, const CommView *comm = nullptr);
 constexpr int TTQ_TRACE_ENTRIES = 8192;

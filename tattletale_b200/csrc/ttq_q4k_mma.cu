@@ -721,6 +721,18 @@ cudaError_t qm_dispatch(const QmParams &p, int sms, size_t ws_bytes, int64_t cou
 
 }  // namespace
 
+// Every CTA converts the rows of its K slice: the gated form computes silu(gate) * up once per CTA where a separate pass does it
+// once.  Where K is not split, the pass (a launch, about 2 us) pays from about 25 K values of the rows.  Measured with the gate|up
+// projection before it, us, gated against separate (hidden, ffn): 2048, 6144 at 4 rows 25.1 / 25.3, at 5 28.3 / 27.7, at 8 34.3 /
+// 30.5; 2048, 4096 at 6 rows 23.6 / 24.1, at 8 27.1 / 26.5; 4096, 14336 at 3 rows 56.6 / 52.2.  With K split the gated form is
+// ahead (4096, 14336 at 5 rows 55.0 / 56.3; 2048, 8192 at 8 rows 28.8 / 31.1), and so it is at 9 rows and more.
+bool q4k_mma_gated_pays(const LinearArgs &a, int sms, size_t ws_bytes, int64_t counters_cap) {
+    QmPlan plan;
+    const bool found = a.M <= 8 ? qm_plan<F16Backend<1, 16>>(a, sms, ws_bytes, counters_cap, plan) : qm_plan<F16Backend<2, 20>>(a, sms, ws_bytes, counters_cap, plan);
+    if (!found || plan.ksplit > 1) return true;
+    return a.M * a.K <= 25600;
+}
+
 bool q4k_mma_supported(const LinearArgs &a) {
     return a.M >= 1 && a.M <= QM_MAX_M && (a.x_dt == TTQ_DT_BF16 || a.x_dt == TTQ_DT_F16) && a.K == a.SBp * TILE_K;
 }

@@ -371,10 +371,13 @@ class GatedMLP:
         gate_up = self.gate_up_proj.forward(x)
         if self.activation != ActivationKind.kSilu:
             raise TtqError(3, f"activation {self.activation} is not implemented")
-        if self.down_proj.fmt == _lib.FMT_TQ3:
-            return self.down_proj.forward(silu_and_mul(self.ctx, gate_up))
-        # the activation inside the down projection's input conversion: one pass over gate|up and one rounding less
-        return self.down_proj.forward_gated(gate_up)
+        down = self.down_proj
+        rows = gate_up.numel() // (2 * down.in_features)
+        # the activation inside the down projection's input conversion: one pass over gate|up and one rounding less (one row or many
+        # always gain by it)
+        if down.fmt != _lib.FMT_TQ3 and (rows == 1 or rows > 16 or self.ctx._lib.ttq_linear_gated_pays(self.ctx.handle, down.handle, rows)):
+            return down.forward_gated(gate_up)
+        return down.forward(silu_and_mul(self.ctx, gate_up))
 
     __call__ = forward
 

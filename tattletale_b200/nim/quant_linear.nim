@@ -50,6 +50,7 @@ proc ttq_silu_and_mul(ctx: ptr TtqCtx, inp: pointer, dt: TtqDtype, M, H, ldIn: i
 proc ttq_linear_forward_gated(ctx: ptr TtqCtx, w: ptr TtqWeight, gateUp: pointer, xDt: TtqDtype, M, ldGateUp: int64,
                               bias: pointer, biasDt: TtqDtype, y: pointer, yDt: TtqDtype, ldy: int64,
                               stream: pointer): TtqStatus {.importc, cdecl, header: "ttq.h".}
+proc ttq_linear_gated_pays(ctx: ptr TtqCtx, w: ptr TtqWeight, M: int64): int32 {.importc, cdecl, header: "ttq.h".}
 proc ttq_add_rmsnorm(ctx: ptr TtqCtx, h, delta, weight: pointer, dt: TtqDtype, M, H, ldH, ldDelta: int64,
                      eps: cfloat, outp: pointer, ldOut: int64, stream: pointer): TtqStatus {.importc, cdecl, header: "ttq.h".}
 proc ttq_add_rmsnorm_prepare(ctx: ptr TtqCtx, h, delta, weight: pointer, dt: TtqDtype, M, H, ldH, ldDelta: int64,

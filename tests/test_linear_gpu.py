@@ -335,3 +335,21 @@ def test_gated_input_conversion(ctx, fmt, m):
     with pytest.raises(ttq.TtqError):
         lin.forward_gated(gu.cuda()[:, : k])
     lin.close()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 6, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("hidden,inter", [(256, 1024), (512, 4096)])
+def test_gated_mlp_takes_the_faster_form(ctx, hidden, inter, m):
+    """GatedMLP on Q4_K: the fused activation where ttq_linear_gated_pays says so, else silu_and_mul and the plain projection; either
+    way exactly those calls."""
+    weights = [torch.from_numpy(make_weight(ttq.FMT_Q4_K, n, k, seed=n + k + i)) for i, (n, k) in enumerate([(inter, hidden), (inter, hidden), (hidden, inter)])]
+    mlp = ttq.GatedMLP(ctx, ttq.FMT_Q4_K, *weights, hidden, inter)
+    x = make_x(m, hidden, seed=m).cuda()
+    down = mlp.down_proj
+    pays = bool(ctx._lib.ttq_linear_gated_pays(ctx.handle, down.handle, m))
+    # up to 25600 values of the rows where K is not split (4096: it is from 9 rows)
+    assert pays == (inter == 1024 or m not in (7, 8))
+    gate_up = mlp.gate_up_proj.forward(x)
+    want = down.forward_gated(gate_up) if pays else down.forward(ttq.silu_and_mul(ctx, gate_up))
+    assert torch.equal(mlp.forward(x), want)
+    ctx.check_device_status()
