@@ -1430,7 +1430,8 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
     // a CTA with two sub-tiles does twice the work per activation stage in about 1.65x the time of one (measured: five
     // rounds of one sub-tile against three of two on 4096 -> 28672 at 768 rows take 221 against 203 us; the single
     // sub-tile is expanded by two warp groups on alternating stages)
-    // TTQ_GEMM_PAIR: 0 never, 1 (default) where the model prefers it, 2 wherever it applies
+    // TTQ_GEMM_PAIR: 0 never, 1 (default) where the model prefers it, 2 wherever it applies (dense Q4_K, more than 128 rows and 128
+    // output features; K is not split then)
     static const int pair_mode = []() {
         const char *v = getenv("TTQ_GEMM_PAIR");
         return v ? atoi(v) : 1;
@@ -1449,6 +1450,8 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
         if (slots > 0 && tiles2 > sms / 2 && pair_makespan((a.N + 255) / 256, mp / 512, mp % 512 ? 1 : 0, slots, iters, true) < cost1 * (iters + 8.0) / 1.65)
             nsub = 2;
     }
+    const bool force_pair = pair_mode >= 2 && !plain && fmt == TTQ_FMT_Q4_K && BM == 256 && a.N > 128 && pair_slots(sms) > 0;
+    if (force_pair) nsub = 2;
     if (plain || fmt != TTQ_FMT_Q4_K) nsub = 2;  // plain: no conversion work to balance; Q8_0 / Q6_K: one variant
     int64_t slab = (xh_capacity / Kp) / BM * BM;  // rows per pass
     if (slab < BM) return cudaErrorInvalidValue;
@@ -1485,7 +1488,7 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
             const int64_t tiles = ((a.N + 128 * nsub - 1) / (128 * nsub)) * m_tiles;
             const size_t xh_bytes = (size_t)Mp * Kp * sizeof(__half);
             const size_t ws_cap = (size_t)xh_capacity * sizeof(__half) > xh_bytes ? (size_t)xh_capacity * sizeof(__half) - xh_bytes : 0;
-            for (int cand = 2; cand <= 8; cand++) {
+            for (int cand = 2; cand <= 8 && !force_pair; cand++) {
                 if (a.SBp % cand || a.SBp / cand < 2) continue;
                 if (tiles * cand > sms) break;
                 if ((size_t)cand * Mp * a.N * sizeof(float) > ws_cap) break;
