@@ -1421,7 +1421,8 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
     if (!plain && !gemm_supported(fmt)) return cudaErrorNotSupported;
     const int kmap = (!plain && fmt == TTQ_FMT_Q6_K) ? 1 : 0;
     const int64_t Kp = a.SBp * TILE_K;
-    const int BM = a.M <= 64 ? 64 : (a.M <= 128 ? 128 : 256);
+    // (up to 192 rows the block formats run ttq_gemm_ts.cu)
+    const int BM = !plain ? 256 : (a.M <= 64 ? 64 : (a.M <= 128 ? 128 : 256));
     // two 128-row sub-tiles per CTA once there are enough tiles to keep every SM busy with them
     static const int force_nsub = []() {
         const char *v = getenv("TTQ_GEMM_NSUB");
@@ -1504,26 +1505,11 @@ cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_cap
                 if (BM == 128) return launch_cfg<128, 2, GM_PLAIN>(q, sms, st);
                 return launch_cfg<256, 2, GM_PLAIN>(q, sms, st);
             }
-            if (fmt == TTQ_FMT_Q8_0) {
-                // (these formats always take two sub-tiles: the single sub-tile variant pays off on the many small tiles
-                // of the grouped Q4_K GEMM, which they do not serve)
-                if (BM == 64) return launch_cfg<64, 2, GM_Q8_0>(q, sms, st);
-                if (BM == 128) return launch_cfg<128, 2, GM_Q8_0>(q, sms, st);
-                return launch_cfg<256, 2, GM_Q8_0>(q, sms, st);
-            }
-            if (fmt == TTQ_FMT_Q6_K) {
-                if (BM == 64) return launch_cfg<64, 2, GM_Q6K>(q, sms, st);
-                if (BM == 128) return launch_cfg<128, 2, GM_Q6K>(q, sms, st);
-                return launch_cfg<256, 2, GM_Q6K>(q, sms, st);
-            }
-            if (nsub == 2) {
-                if (BM == 64) return launch_cfg<64, 2>(q, sms, st);
-                if (BM == 128) return launch_cfg<128, 2>(q, sms, st);
-                return launch_cfg<256, 2>(q, sms, st);
-            }
-            if (BM == 64) return launch_cfg<64, 1>(q, sms, st);
-            if (BM == 128) return launch_cfg<128, 1>(q, sms, st);
-            return launch_cfg<256, 1>(q, sms, st);
+            // (Q8_0 and Q6_K always take two sub-tiles: the single sub-tile variant pays off on the many small tiles of the
+            // grouped Q4_K GEMM, which they do not serve)
+            if (fmt == TTQ_FMT_Q8_0) return launch_cfg<256, 2, GM_Q8_0>(q, sms, st);
+            if (fmt == TTQ_FMT_Q6_K) return launch_cfg<256, 2, GM_Q6K>(q, sms, st);
+            return nsub == 2 ? launch_cfg<256, 2>(q, sms, st) : launch_cfg<256, 1>(q, sms, st);
         };
         auto reduce = [&](const GemmParams &q) -> cudaError_t {
             const int64_t total = (Ms * ((q.N + 3) / 4) + 255) / 256;
