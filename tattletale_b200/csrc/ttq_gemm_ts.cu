@@ -56,8 +56,8 @@ struct TsParams {
     int64_t N, NT;
     int SBp;
     const __half *xh;  // activation images, see launch_xh_images
-    int M, Mp;         // activation rows; image rows = mbs * nb
-    int nb, mbs;       // rows per block (a multiple of 16, at most 256), blocks
+    int M, Mp;         // activation rows; image rows
+    int nb;            // rows per block (a multiple of 16, at most 256); one block, grouped: one per row tile
     const void *bias;
     int bias_dt;
     void *y;
@@ -357,8 +357,8 @@ __device__ __forceinline__ void ts_expand(uint32_t stage, uint32_t hdr, int lane
     }
 }
 
-// Position of an item: tile = outer * ni + inner, super-block.  Dense: outer = 128 weight rows, inner = activation block (the
-// blocks of one run of weights are neighbours); grouped: outer = row tile, inner = 128 weight rows of its expert.
+// Position of an item: tile = outer * ni + inner, super-block.  Dense: outer = 128 weight rows, ni = 1; grouped: outer = row tile,
+// inner = 128 weight rows of its expert.
 struct TsCursor {
     int64_t outer;
     int inner, sb;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    const int nb = p.nb, mbs = p.mbs, SBp = p.SBp, ring = p.ring, bslots = p.bslots;
+    const int nb = p.nb, SBp = p.SBp, ring = p.ring, bslots = p.bslots;
     const uint32_t slice_bytes = (uint32_t)nb * 128u;
     const int spb = p.spb;
     const uint32_t b_u32 = base, ring_u32 = b_u32 + bslots * spb * slice_bytes, hdr_u32 = ring_u32 + TS_CONV_WARPS * ring * TB;
@@ -412,11 +412,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         if (T < G) G = T;
         if ((int64_t)blockIdx.x >= G) return;  // fewer items than CTAs: the last ones have none
     }
-    const int ni = grouped ? (int)((p.N + TS_ROWS - 1) / TS_ROWS) : mbs;
+    const int ni = grouped ? (int)((p.N + TS_ROWS - 1) / TS_ROWS) : 1;
     auto group_of = [&](const TsCursor &c) -> int64_t { return grouped ? (int64_t)c.inner : c.outer; };
-    // first image row of a block, and how many of its rows exist
-    auto row0_of = [&](const TsCursor &c) -> int { return grouped ? p.mt_row0[c.outer] : c.inner * nb; };
-    auto rows_of = [&](const TsCursor &c) -> int { return grouped || p.M - c.inner * nb >= nb ? nb : p.M - c.inner * nb; };
+    // first image row of a block
+    auto row0_of = [&](const TsCursor &c) -> int { return grouped ? p.mt_row0[c.outer] : 0; };
+    const int rows = grouped ? nb : p.M;  // of a block's rows, those that exist
     const int64_t i0 = (int64_t)blockIdx.x * T / G;
     const int n_items = (int)(((int64_t)blockIdx.x + 1) * T / G - i0);
     const int64_t first_tile = i0 / SBp;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             const bool whole = run == SBp;
             const int buf = seg % nd, use = seg / nd;
             const int64_t tile = c.outer * ni + c.inner;
-            const int rows = rows_of(c), row0 = row0_of(c);
+            const int row0 = row0_of(c);
             unsigned others = 0;  // CTAs besides this one that hold a piece of the tile
             if (!whole && threadIdx.x == 0) others = (unsigned)(((tile + 1) * SBp * G - 1) / T - ((tile * SBp + 1) * G - 1) / T);
             if (alive) alive = ts_wait_warp(d_full + 8 * buf, (uint32_t)(use & 1), p.status, lane);
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                 const uint32_t dst = b_u32 + (uint32_t)(slot * spb) * slice_bytes, bar = b_full + 8 * slot;
                 if (alive && ts_elect()) {
                     mbar_expect_tx(bar, spb * slice_bytes);
-                    if (p.Mp == nb) {
+                    if (!grouped) {
                         bulk_g2s(dst, from + n * it_stride, spb * slice_bytes, bar);  // the slices of one block are neighbours
                     } else {
                         for (int q = 0; q < spb; q++) bulk_g2s(dst + q * slice_bytes, from + (n + q) * it_stride, slice_bytes, bar);
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         TsCursor c;
         c.init(tile * SBp, SBp, ni);
         const int64_t group = group_of(c);
-        const int rows = rows_of(c), row0 = row0_of(c);
+        const int row0 = row0_of(c);
         const size_t piece = (size_t)nb * TS_ROWS;
         // the first CTA of the tile parked its piece in its second slot, unless its own run starts inside the tile; every
         // other one in its first slot
@@ -812,21 +812,19 @@ cudaError_t ts_launch(TsParams &p, int grid, cudaStream_t st) {
 cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                            int64_t counters_cap, cudaStream_t st, int *launches) {
     *launches = 0;
-    if (!gemm_supported(fmt) || a.M < 1) return cudaErrorNotSupported;
+    if (!gemm_supported(fmt) || a.M < 1 || a.M > 256) return cudaErrorNotSupported;
     TsParams p;
-    p.mbs = (int)((a.M + 255) / 256);
-    p.nb = (int)(((a.M + p.mbs - 1) / p.mbs + 15) / 16 * 16);
     p.M = (int)a.M;
-    p.Mp = p.mbs * p.nb;
+    p.nb = p.Mp = (p.M + 15) / 16 * 16;
     p.tiles = a.tiles;
     p.N = a.N; p.NT = a.NT; p.SBp = (int)a.SBp;
     const int64_t groups = (a.N + TS_ROWS - 1) / TS_ROWS;
-    p.T = groups * p.mbs * a.SBp;
-    const int grid = ts_grid(p.T, groups * p.mbs, p.SBp, p.nb, sms);
+    p.T = groups * a.SBp;
+    const int grid = ts_grid(p.T, groups, p.SBp, p.nb, sms);
     const int64_t Kp = a.SBp * TILE_K;
     const size_t xh_bytes = ((size_t)p.Mp * Kp * sizeof(__half) + 255) & ~(size_t)255;
     const size_t ws_bytes = (size_t)2 * grid * p.nb * TS_ROWS * sizeof(float);
-    if (xh_bytes + ws_bytes > (size_t)xh_capacity * sizeof(__half) || groups * p.mbs > counters_cap) return cudaErrorNotSupported;
+    if (xh_bytes + ws_bytes > (size_t)xh_capacity * sizeof(__half) || groups > counters_cap) return cudaErrorNotSupported;
     p.xh = xh;
     p.ws = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xh) + xh_bytes);
     p.counters = counters;
@@ -913,7 +911,7 @@ cudaError_t launch_gemm_ts_precise(int fmt, const LinearArgs &a, const float *to
     constexpr int NB = TS_PRECISE_ROWS;
     if ((fmt != TTQ_FMT_Q8_0 && fmt != TTQ_FMT_Q6_K) || a.M < 1 || a.M > NB || a.gated) return cudaErrorNotSupported;
     TsParams p;
-    p.mbs = 1; p.nb = NB;
+    p.nb = NB;
     p.M = (int)a.M; p.Mp = NB;
     p.tiles = a.tiles;
     p.N = a.N; p.NT = a.NT; p.SBp = (int)a.SBp;
@@ -952,7 +950,7 @@ bool gemm_ts_grouped_fits(const GroupedArgs &g, int sms) {
 cudaError_t launch_gemm_ts_grouped(const GroupedArgs &g, const __half *xh, int sms, int *status, cudaStream_t st) {
     if (!gemm_ts_grouped_fits(g, sms)) return cudaErrorInvalidValue;
     TsParams p;
-    p.nb = g.BM; p.mbs = 1;
+    p.nb = g.BM;
     p.M = (int)g.Mp; p.Mp = (int)g.Mp;
     p.tiles = nullptr;
     p.N = g.N; p.NT = g.NT; p.SBp = (int)g.SBp;

@@ -333,7 +333,7 @@ bool gemm_supported(int fmt);
 // `wimg` != nullptr selects the plain mode: both operands are fp16 tile images (the trellis format's expansion).
 cudaError_t launch_gemm(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status,
                         unsigned long long *trace, cudaStream_t st, int *launches, const __half *wimg = nullptr);
-// Batches of one or a few 256-row blocks: weights expanded into tensor memory (ttq_gemm_ts.cu); formats as gemm_supported.
+// Batches of up to 256 rows: weights expanded into tensor memory (ttq_gemm_ts.cu); formats as gemm_supported.
 // `counters` are zero between launches.  cudaErrorNotSupported: the caller takes another path.
 cudaError_t launch_gemm_ts(int fmt, const LinearArgs &a, __half *xh, int64_t xh_capacity, int sms, int *status, unsigned *counters,
                            int64_t counters_cap, cudaStream_t st, int *launches);
