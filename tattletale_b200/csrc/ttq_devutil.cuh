@@ -1,4 +1,4 @@
-// Device-side helpers shared by the decode kernels: bulk-copy rings on mbarriers (every wait bounded),
+// Device-side helpers shared by the kernels: bulk-copy rings on mbarriers (every wait bounded),
 // shared-memory access with immediate offsets, the per-kernel timeline entry, a compile-time loop.
 #pragma once
 
@@ -43,6 +43,57 @@ __device__ __forceinline__ void named_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---- tensor-core pipelines (tcgen05) -------------------------------------------------------------
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+constexpr int TC_WAIT_LIMIT = 1 << 22;
+// Bounded wait of the tensor-core pipelines: after TC_WAIT_LIMIT polls the failure is recorded and the caller carries on (with
+// garbage data) so that every role still finishes and tensor memory is released.
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, int *status) {
+    for (int i = 0; i < TC_WAIT_LIMIT; i++)
+        if (mbar_try_wait(bar, parity)) return true;
+    report_failure(status, 2);
+    return false;
+}
+// Warp-wide form: lane 0 polls, the others park at the warp barrier (fewer shared-memory polls next to the
+// tensor core's operand reads).
+__device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, int *status, int lane) {
+    bool ok = true;
+    if (lane == 0) ok = tc_wait(bar, parity, status);
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+}
+// One lane of a converged warp.  tcgen05.mma and bulk copies issued by an elected lane of a warp that walks its loop as a whole took
+// 17 cycles each (N = 16; the tensor core's own time from N = 64), from a branch on the lane number about 100.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes,
+// 8-row atoms of 1024 bytes stacked contiguously (stride byte offset 1024), descriptor version 1.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
+    const uint32_t lo = ((addr & 0x3ffffu) >> 4) | (1u << 16);          // start address, leading byte offset (unused) = 1
+    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);         // stride byte offset, version = 1, SWIZZLE_128B
+    return ((uint64_t)hi << 32) | lo;
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// Half h of a Q4_K row header's 6-bit fields, four to a word: scales and mins of sub-blocks 4h .. 4h + 3.
+__device__ __forceinline__ void q4k_scale_words(const uint4 &hv, int h, uint32_t &scales, uint32_t &mins) {
+    if (h == 0) {
+        scales = hv.y & 0x3f3f3f3fu;
+        mins = hv.z & 0x3f3f3f3fu;
+    } else {
+        scales = (hv.w & 0x0f0f0f0fu) | ((hv.y >> 2) & 0x30303030u);
+        mins = ((hv.w >> 4) & 0x0f0f0f0fu) | ((hv.z >> 2) & 0x30303030u);
+    }
+}
 
 // ---- timeline -----------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long global_ns() {

@@ -29,7 +29,7 @@
 // tables.  Every mbarrier wait is bounded; tensor memory is always released.
 #include <cstdlib>
 
-#include "ttq_internal.cuh"
+#include "ttq_devutil.cuh"
 
 namespace ttq {
 
@@ -43,64 +43,7 @@ __host__ __device__ constexpr int gemm_deq_warps(int) { return 16; }
 __host__ __device__ constexpr int gemm_warps(int nsub) { return GEMM_EPI_WARPS + gemm_deq_warps(nsub) + 1; }
 constexpr int GEMM_BN = 128;                     // weight rows per CTA = MMA M
 constexpr int A_STAGE_BYTES = GEMM_BN * 128;     // 128 rows x 64 fp16
-constexpr int GEMM_WAIT_LIMIT = 1 << 22;
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: after GEMM_WAIT_LIMIT polls the failure is recorded and the caller carries on (with
-// garbage data) so that every role still finishes and tensor memory is released.
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, int *status) {
-    for (int i = 0; i < GEMM_WAIT_LIMIT; i++)
-        if (mbar_try_wait(bar, parity)) return true;
-    report_failure(status, 2);
-    return false;
-}
-// Warp-wide form: lane 0 polls, the others park at the warp barrier (fewer shared-memory polls next to the
-// tensor core's operand reads).
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int *status, int lane) {
-    bool ok = true;
-    if (lane == 0) ok = mbar_wait_bounded(bar, parity, status);
-    __syncwarp();
-    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes,
-// 8-row atoms of 1024 bytes stacked contiguously (stride byte offset 1024), descriptor version 1.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    const uint32_t lo = ((addr & 0x3ffffu) >> 4) | (1u << 16);          // start address, leading byte offset (unused) = 1
-    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);         // stride byte offset, version = 1, SWIZZLE_128B
-    return ((uint64_t)hi << 32) | lo;
-}
 // Instruction descriptor, kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = n.
 __host__ __device__ constexpr uint32_t idesc_f16(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24); }
 
@@ -113,17 +56,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
         "}\n" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
-}
-// One lane of a converged warp.  tcgen05.mma and bulk copies take their operands from uniform registers: issued by an elected
-// lane of a warp that walks its loop as a whole they are one instruction each (17 cycles for N = 16, the tensor core's own
-// time from N = 64), from a branch on the lane number the compiler makes a loop of about 100 cycles of each.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
-    return e != 0;
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -357,7 +289,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
             mbar_init(acce_bar + 8 * b, GEMM_EPI_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fence_async_smem();
+        fence_async_shared();
     }
     if (warp == C::WARPS - 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_slot)),
@@ -379,7 +311,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
             const int64_t otile = tile / splits, split = tile % splits;
             const int64_t n_tile = tile_n(otile), m_tile = tile_m(otile);
             const int buf = tcount % C::NACC, use = tcount / C::NACC;
-            if (alive) alive = mbar_wait_warp(accf_bar + 8 * buf, (uint32_t)(use & 1), p.status, lane);
+            if (alive) alive = tc_wait_warp(accf_bar + 8 * buf, (uint32_t)(use & 1), p.status, lane);
             tc_fence_after();
             const int64_t m0 = tile_row0(m_tile);
             const int mh = tile_mh(m_tile);
@@ -465,7 +397,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (git >= STAGES && alive)
-                        alive = mbar_wait_bounded(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status);
+                        alive = tc_wait(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status);
                     const uint32_t a_stage = stages_u32 + stage * C::STAGE_BYTES;
                     if (elect_one()) {
                         mbar_expect_tx(full_bar + 8 * stage, C::A_BYTES + C::B_BYTES);
@@ -615,13 +547,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                             const __half2 dd = *reinterpret_cast<const __half2 *>(&hv.x);
                             const float d = __low2float(dd), dmin = __high2float(dd);
                             uint32_t scw, mw;
-                            if (h == 0) {
-                                scw = hv.y & 0x3f3f3f3fu;
-                                mw = hv.z & 0x3f3f3f3fu;
-                            } else {
-                                scw = (hv.w & 0x0f0f0f0fu) | ((hv.y >> 2) & 0x30303030u);
-                                mw = ((hv.w >> 4) & 0x0f0f0f0fu) | ((hv.z >> 2) & 0x30303030u);
-                            }
+                            q4k_scale_words(hv, h, scw, mw);
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
                                 const float sc = d * (float)((scw >> (8 * i)) & 0xff);
@@ -662,7 +588,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 }
                 unsigned long long tw0 = trd ? global_ns() : 0;
                 if (git >= STAGES && alive)
-                    alive = mbar_wait_warp(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status, lane);
+                    alive = tc_wait_warp(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status, lane);
                 if (trd) {
                     tw0 = global_ns() - tw0;
                     t_empty += tw0;
@@ -754,7 +680,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                                      : "memory");
                     }
                 }
-                fence_async_smem();
+                fence_async_shared();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_bar + 8 * stage);
                 if (trd) t_conv += global_ns() - tw0;
@@ -787,7 +713,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 const int buf = tcount % C::NACC, use = tcount / C::NACC;
                 // the epilogue must have drained this accumulator set (its previous use)
                 unsigned long long t0 = tr ? global_ns() : 0;
-                if (use >= 1 && alive) alive = vote(mbar_wait_bounded(acce_bar + 8 * buf, (uint32_t)((use - 1) & 1), p.status));
+                if (use >= 1 && alive) alive = vote(tc_wait(acce_bar + 8 * buf, (uint32_t)((use - 1) & 1), p.status));
                 if (tr) t_acc += global_ns() - t0;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS);
@@ -795,7 +721,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, NSUB>::THREADS, 1) gemm_q4k_kernel
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (tr) t0 = global_ns();
-                    if (alive) alive = vote(mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
+                    if (alive) alive = vote(tc_wait(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
                     if (tr) {
                         t_full += global_ns() - t0;
                         t0 = global_ns();
@@ -887,7 +813,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t rank)
 }
 // bounded wait with cluster-scope acquire: the arrivals it observes come from both CTAs of the pair
 __device__ __forceinline__ bool mbar_wait_bounded_cluster(uint32_t bar, uint32_t parity, int *status) {
-    for (int i = 0; i < GEMM_WAIT_LIMIT; i++) {
+    for (int i = 0; i < TC_WAIT_LIMIT; i++) {
         uint32_t ok;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -958,7 +884,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
         mbar_init(accf_bar, 1);
         mbar_init(acce_bar, 2 * GP_EPI_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fence_async_smem();
+        fence_async_shared();
     }
     if (warp == GP_WARPS - 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_slot)), "r"(512u) : "memory");
@@ -979,7 +905,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
         for (int64_t tile = pair; tile < n_otiles; tile += n_pairs, tcount++) {
             int64_t n_tile, m_tile;
             const int mh = tile_at(tile, n_tile, m_tile);
-            if (alive) alive = mbar_wait_warp(accf_bar, (uint32_t)(tcount & 1), p.status, lane);
+            if (alive) alive = tc_wait_warp(accf_bar, (uint32_t)(tcount & 1), p.status, lane);
             tc_fence_after();
             const int quad = warp & 3;  // a warp reads the 32 tensor-memory lanes of its quarter
             const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -1116,13 +1042,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                     const __half2 dd = *reinterpret_cast<const __half2 *>(&hv.x);
                     const float d = __low2float(dd), dmin = __high2float(dd);
                     uint32_t scw, mw;
-                    if (h == 0) {
-                        scw = hv.y & 0x3f3f3f3fu;
-                        mw = hv.z & 0x3f3f3f3fu;
-                    } else {
-                        scw = (hv.w & 0x0f0f0f0fu) | ((hv.y >> 2) & 0x30303030u);
-                        mw = ((hv.w >> 4) & 0x0f0f0f0fu) | ((hv.z >> 2) & 0x30303030u);
-                    }
+                    q4k_scale_words(hv, h, scw, mw);
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const float sc = d * (float)((scw >> (8 * i)) & 0xff);
@@ -1136,7 +1056,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                     __syncwarp();
                 }
                 unsigned long long tw0 = trd ? global_ns() : 0;
-                if (git >= STAGES && alive) alive = mbar_wait_warp(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status, lane);
+                if (git >= STAGES && alive) alive = tc_wait_warp(empty_bar + 8 * stage, (uint32_t)(((git / STAGES) - 1) & 1), p.status, lane);
                 if (trd) {
                     t_empty += global_ns() - tw0;
                     tw0 = global_ns();
@@ -1180,7 +1100,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                                      : "memory");
                     }
                 }
-                fence_async_smem();  // (both CTAs' tensor cores read these rows; the release at cluster scope below orders them)
+                fence_async_shared();  // (both CTAs' tensor cores read these rows; the release at cluster scope below orders them)
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive((rank == 0 ? full_bar : act_bar) + 8 * stage);
@@ -1219,7 +1139,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
                     if (tr) t0 = global_ns();
-                    if (alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
+                    if (alive) alive = __all_sync(0xffffffffu, tc_wait(full_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status));
                     if (tr) {
                         t_full += global_ns() - t0;
                         t0 = global_ns();
@@ -1260,7 +1180,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_q4k_pair_kernel(GemmParams
             for (int64_t tile = pair; tile < n_otiles; tile += n_pairs) {
                 for (int it = 0; it < iters; it++, git++) {
                     const int stage = git % STAGES;
-                    if (alive) alive = mbar_wait_bounded(act_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status);
+                    if (alive) alive = tc_wait(act_bar + 8 * stage, (uint32_t)((git / STAGES) & 1), p.status);
                     mbar_arrive_cluster(full_bar + 8 * stage, 0);
                 }
             }

@@ -49,7 +49,6 @@ constexpr int TS_MAX_A = 3;  // A stages in tensor memory
 constexpr int TS_BAR_BYTES = (TS_CONV_WARPS * TS_MAX_RING + 2 * TS_MAX_BSLOTS + 2 * TS_MAX_A + 4) * 8 + 32;
 constexpr int TS_SMEM_MAX = 227 * 1024;
 constexpr int TS_A_COLS = 128, TS_TMEM_COLS = 512;
-constexpr int TS_WAIT_LIMIT = 1 << 22;
 
 struct TsParams {
     const uint8_t *tiles;
@@ -78,32 +77,6 @@ struct TsParams {
     const float *top;        // exact form: Weight::top
 };
 
-__device__ __forceinline__ void ts_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool ts_wait(uint32_t bar, uint32_t parity, int *status) {
-    for (int i = 0; i < TS_WAIT_LIMIT; i++)
-        if (mbar_try_wait(bar, parity)) return true;
-    report_failure(status, 2);
-    return false;
-}
-__device__ __forceinline__ bool ts_wait_warp(uint32_t bar, uint32_t parity, int *status, int lane) {
-    bool ok = true;
-    if (lane == 0) ok = ts_wait(bar, parity, status);
-    __syncwarp();
-    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-}
-__device__ __forceinline__ void ts_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void ts_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ bool ts_elect() {
-    uint32_t e;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
-    return e != 0;
-}
-// K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row atoms of 1024 bytes stacked contiguously
-__device__ __forceinline__ uint64_t ts_desc_sw128(uint32_t addr) {
-    const uint32_t lo = ((addr & 0x3ffffu) >> 4) | (1u << 16);
-    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-    return ((uint64_t)hi << 32) | lo;
-}
 // kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t ts_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24); }
 __device__ __forceinline__ void ts_mma(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -115,9 +88,6 @@ __device__ __forceinline__ void ts_mma(uint32_t d, uint32_t a, uint64_t bdesc, u
         "}\n" ::"r"(d),
         "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-__device__ __forceinline__ void ts_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void ts_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -176,13 +146,7 @@ __device__ __forceinline__ void ts_header(uint32_t stage, uint32_t hdr, int lane
         const __half2 dd = ts_as_h2(hv.x);
         const float d = __low2float(dd), dmin = __high2float(dd);
         uint32_t scw, mw;
-        if (h == 0) {
-            scw = hv.y & 0x3f3f3f3fu;
-            mw = hv.z & 0x3f3f3f3fu;
-        } else {
-            scw = (hv.w & 0x0f0f0f0fu) | ((hv.y >> 2) & 0x30303030u);
-            mw = ((hv.w >> 4) & 0x0f0f0f0fu) | ((hv.z >> 2) & 0x30303030u);
-        }
+        q4k_scale_words(hv, h, scw, mw);
         uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -454,12 +418,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     };
     auto issue_next = [&]() {
         const uint32_t bar = my_bar + 8 * i_stage;
-        if (ts_elect()) {
+        if (elect_one()) {
             if (src_ptr != nullptr) {
                 mbar_expect_tx(bar, TB);
                 bulk_g2s(my_ring + (uint32_t)(i_stage * TB), src_ptr, TB, bar);
             } else {
-                ts_arrive(bar);
+                mbar_arrive(bar);
             }
         }
         issued++;
@@ -475,7 +439,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
     const float top = precise ? __ldcg(p.top) : 0.f;  // on its way beside the first packed tiles, first looked at with them
     if (my_count > 0) {
         // the packed weights depend on no preceding kernel: the ring fills while that one drains
-        if (ts_elect()) {
+        if (elect_one()) {
             for (int s = 0; s < ring; s++) mbar_init(my_bar + 8 * s, 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             fence_async_shared();
@@ -492,9 +456,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    ts_fence_before();
+    tc_fence_before();
     __syncthreads();
-    ts_fence_after();
+    tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp < TS_EPI_WARPS) {
@@ -513,8 +477,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             const int row0 = row0_of(c);
             unsigned others = 0;  // CTAs besides this one that hold a piece of the tile
             if (!whole && threadIdx.x == 0) others = (unsigned)(((tile + 1) * SBp * G - 1) / T - ((tile * SBp + 1) * G - 1) / T);
-            if (alive) alive = ts_wait_warp(d_full + 8 * buf, (uint32_t)(use & 1), p.status, lane);
-            ts_fence_after();
+            if (alive) alive = tc_wait_warp(d_full + 8 * buf, (uint32_t)(use & 1), p.status, lane);
+            tc_fence_after();
             const int64_t n = group_of(c) * TS_ROWS + r;
             const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(d_col + buf * nb);
             const int slot = 2 * (int)blockIdx.x + (tile == first_tile ? 0 : 1);
@@ -538,9 +502,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                         if (c0 + i < rows) __stcg(wsp + (c0 + i) * TS_ROWS, __uint_as_float(v[i]));
                 }
             }
-            ts_fence_before();
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) ts_arrive(d_empty + 8 * buf);
+            if (lane == 0) mbar_arrive(d_empty + 8 * buf);
             if (!whole) {
                 named_barrier(1, TS_EPI_WARPS * 32);
                 if (threadIdx.x == 0) {
@@ -582,15 +546,15 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             // (exact form: the item takes two A stages, each two slices as rounded weights and remainders)
 #pragma unroll 1
             for (int half = 0; half < (precise ? 2 : 1); half++) {
-                if (a_round >= 1 && alive) alive = ts_wait_warp(a_empty + 8 * as, (uint32_t)((a_round - 1) & 1), p.status, lane);
-                ts_fence_after();
+                if (a_round >= 1 && alive) alive = tc_wait_warp(a_empty + 8 * as, (uint32_t)((a_round - 1) & 1), p.status, lane);
+                tc_fence_after();
                 if (have) {
                     ts_expand<FMT, MODE>(stage, hdr, lane, taddr + (uint32_t)(as * TS_A_COLS), 2 * half);
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 }
-                ts_fence_before();
+                tc_fence_before();
                 __syncwarp();  // also: every lane has read the stage and the records
-                if (lane == 0) ts_arrive(a_full + 8 * as);
+                if (lane == 0) mbar_arrive(a_full + 8 * as);
                 // the next stage of this set: two items on (dense); the item's second stage, then past the other set's two (exact)
                 as += precise ? (half == 0 ? 1 : 3) : 2;
                 while (as >= na) {
@@ -616,17 +580,17 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         const int step = precise ? 2 : spb;  // slices per hand-over (exact form: a whole item per activation slot, two A stages)
         for (int li = 0; li < n_items; li++) {
             const int buf = seg % nd, use = seg / nd;
-            if (fresh && use >= 1 && alive) alive = ts_wait(d_empty + 8 * buf, (uint32_t)((use - 1) & 1), p.status);
+            if (fresh && use >= 1 && alive) alive = tc_wait(d_empty + 8 * buf, (uint32_t)((use - 1) & 1), p.status);
             const uint32_t td = tmem_base + (uint32_t)(d_col + buf * nb);
             const bool done = sb + 1 == SBp || li == n_items - 1;
 #pragma unroll 1
             for (int n = 0; n < 4; n += step) {
-                if ((precise || n == 0) && alive) alive = ts_wait(a_full + 8 * as, apar, p.status);
-                if ((!precise || n == 0) && alive) alive = ts_wait(b_full + 8 * slot, bpar, p.status);
+                if ((precise || n == 0) && alive) alive = tc_wait(a_full + 8 * as, apar, p.status);
+                if ((!precise || n == 0) && alive) alive = tc_wait(b_full + 8 * slot, bpar, p.status);
                 __syncwarp();
-                ts_fence_after();
-                if (ts_elect()) {
-                    uint64_t bd = ts_desc_sw128(b_u32 + (uint32_t)(slot * spb) * slice_bytes + (precise ? (uint32_t)n * slice_bytes : 0u));
+                tc_fence_after();
+                if (elect_one()) {
+                    uint64_t bd = smem_desc_sw128(b_u32 + (uint32_t)(slot * spb) * slice_bytes + (precise ? (uint32_t)n * slice_bytes : 0u));
                     uint32_t ta = tmem_base + (uint32_t)(as * TS_A_COLS + (precise ? 0 : n * 32));
                     for (int q = 0; q < step; q++) {
                         ts_mma(td, ta, bd, idesc, (fresh && n + q == 0) ? 0u : 1u);
@@ -639,9 +603,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
                         ta += 32;
                         bd += (uint64_t)(slice_bytes >> 4);
                     }
-                    if (!precise || n + step == 4) ts_commit(b_empty + 8 * slot);
-                    if (precise || n + step == 4) ts_commit(a_empty + 8 * as);
-                    if (n + step == 4 && done) ts_commit(d_full + 8 * buf);
+                    if (!precise || n + step == 4) umma_commit(b_empty + 8 * slot);
+                    if (precise || n + step == 4) umma_commit(a_empty + 8 * as);
+                    if (n + step == 4 && done) umma_commit(d_full + 8 * buf);
                 }
                 __syncwarp();
                 if ((!precise || n + step == 4) && ++slot == bslots) {
@@ -674,9 +638,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
         for (int li = 0; li < n_items; li++) {
             const uint8_t *from = img + (int64_t)c.sb * 4 * it_stride + (((int64_t)row0_of(c) >> 3) << 10);
             for (int n = 0; n < 4; n += spb, filled++) {
-                if (filled >= bslots && alive) alive = __all_sync(0xffffffffu, ts_wait(b_empty + 8 * slot, par, p.status));
+                if (filled >= bslots && alive) alive = __all_sync(0xffffffffu, tc_wait(b_empty + 8 * slot, par, p.status));
                 const uint32_t dst = b_u32 + (uint32_t)(slot * spb) * slice_bytes, bar = b_full + 8 * slot;
-                if (alive && ts_elect()) {
+                if (alive && elect_one()) {
                     mbar_expect_tx(bar, spb * slice_bytes);
                     if (!grouped) {
                         bulk_g2s(dst, from + n * it_stride, spb * slice_bytes, bar);  // the slices of one block are neighbours
@@ -692,10 +656,10 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const TsParams p
             c.advance(1, SBp, ni);
         }
     }
-    ts_fence_before();
+    tc_fence_before();
     __syncthreads();
     if (warp == TS_MMA_WARP) {
-        ts_fence_after();
+        tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TS_TMEM_COLS) : "memory");
     }
     // ---- the tiles whose last piece came from this CTA: all threads add the pieces, four outputs each, in run order
