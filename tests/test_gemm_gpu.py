@@ -1,4 +1,5 @@
-"""Tensor-core (tcgen05) dequant-GEMM (Q4_K beyond 16 rows, Q8_0 / Q6_K from 9) against the CPU checker, through the C ABI.
+"""Tensor-core (tcgen05) dequant-GEMMs (Q4_K beyond 16 rows, Q8_0 / Q6_K from 9) against the CPU checker, through the C ABI: the
+tensor-memory kernel up to 192 rows (its own edges: test_gemm_ts_gpu.py), the shared-memory kernels beyond.
 
 Weights are expanded to fp16 before the MMA and activations are converted to fp16, so the expected
 relative L2 error is a few 1e-4 (bar: 1e-3, fp32 accumulation in tensor memory)."""
@@ -39,7 +40,7 @@ def test_row_counts(ctx, m):
 
 @pytest.mark.parametrize("n,k", [(128, 256), (100, 512), (130, 768), (16, 256), (384, 2304)])
 def test_ragged_weight_shapes(ctx, n, k):
-    for m in (40, 150):
+    for m in (40, 150, 193, 300):
         got, want = run(ctx, n, k, m, seed=n + k + m)
         assert rel_l2(got, want) < TOL
 
@@ -68,10 +69,11 @@ def test_same_rows_give_same_result_as_decode_path(ctx):
 
 
 @pytest.mark.parametrize("fmt", [ttq.FMT_Q8_0, ttq.FMT_Q6_K], ids=["q8_0", "q6_k"])
-@pytest.mark.parametrize("n,k,m", [(256, 512, 33), (130, 768, 200), (512, 1024, 300), (100, 256, 64), (272, 2304, 9), (4096, 1024, 40)])
+@pytest.mark.parametrize("n,k,m", [(256, 512, 33), (130, 768, 200), (512, 1024, 300), (100, 256, 64), (272, 2304, 9), (4096, 1024, 40),
+                                   (101, 512, 193), (130, 768, 300), (384, 2304, 255)])
 def test_q8_0_and_q6_k_fused_dequant_gemm(ctx, fmt, n, k, m):
-    """Q8_0 and Q6_K batches from 9 rows: the same tcgen05 kernel as Q4_K, its dequant warps expanding int8 values
-    (Q8_0) or nibble + 2-bit planes (Q6_K) to fp16 in shared memory; no whole-weight expansion."""
+    """Q8_0 and Q6_K batches from 9 rows: the same tcgen05 kernels as Q4_K, their conversion warps expanding int8 values
+    (Q8_0) or nibble + 2-bit planes (Q6_K) to fp16 in tensor memory or, beyond 192 rows, shared memory; no whole-weight expansion."""
     from gpu_util import OFMT
 
     blocks = make_weight(fmt, n, k, seed=n + k + m + fmt)
@@ -85,3 +87,13 @@ def test_q8_0_and_q6_k_fused_dequant_gemm(ctx, fmt, n, k, m):
     want = oracle.linear(OFMT[fmt], blocks, x_bits(x), oracle.BF16, bias.numpy())
     assert rel_l2(y.cpu().numpy(), want) < TOL
     lin.close()
+
+
+@pytest.mark.parametrize("n", [129, 130, 131])
+@pytest.mark.parametrize("y_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+def test_sum_of_k_splits_of_odd_widths(ctx, n, y_dtype):
+    """Few output tiles of a long K: the K split's partial sums are added one by one where N is not a multiple of four, with a bias."""
+    c0 = ctx.launch_count
+    got, want = run(ctx, n, 2048, 300, seed=n, y_dtype=y_dtype, bias=True)
+    assert ctx.launch_count - c0 >= 4  # repack, activation images, GEMM, sum
+    assert rel_l2(got, want) < (TOL if y_dtype == torch.float32 else 6e-3)

@@ -1,9 +1,10 @@
 """The GEMM that expands packed weights into tensor memory, at the sizes where its split can go wrong, against the CPU checker.
 
 Row counts around the 16-row granularity of the activation block, the switch from two accumulator sets to one (128) and the
-largest block (256); weight rows that end inside a 16-row tile and inside a 128-row group; one super-block, an odd number,
-and enough to cut every output tile over several CTAs (partial sums and arrival counters: a second call must agree bit for
-bit).  Weights and activations are rounded to fp16 (2^-11 each, independent), sums are fp32: expected relative L2 error
+largest block (256; beyond 192 rows matrices of long K and few weight rows run this kernel: two activation slots of one slice each);
+weight rows that end inside a 16-row tile and inside a 128-row group; one super-block, an odd number, and enough to cut every output
+tile over several CTAs (partial sums and arrival counters: a second call must agree bit for bit).  That this kernel ran shows in the
+number of launches: the shared-memory GEMM would split K on the shapes beyond 192 rows and add a third.  Weights and activations are rounded to fp16 (2^-11 each, independent), sums are fp32: expected relative L2 error
 2e-4 to 4e-4, bar 1e-3."""
 import numpy as np
 import pytest
@@ -20,7 +21,7 @@ TOL = 1e-3
 
 @pytest.mark.parametrize("fmt", ALL_FMTS, ids=FMT_IDS)
 @pytest.mark.parametrize("n,k,m", [(16, 256, 17), (100, 512, 32), (130, 768, 33), (1000, 1024, 48), (256, 2304, 112), (4096, 512, 128),
-                                   (264, 1280, 129), (3000, 2560, 144), (128, 4096, 255), (512, 256, 256)])
+                                   (264, 1280, 129), (3000, 2560, 144), (130, 8192, 193), (264, 8192, 224), (264, 8192, 241), (264, 8192, 256)])
 def test_matches_checker(ctx, fmt, n, k, m):
     dtype = torch.float16 if m % 2 else torch.bfloat16
     blocks = make_weight(fmt, n, k, seed=n + k + m)
@@ -28,7 +29,9 @@ def test_matches_checker(ctx, fmt, n, k, m):
     bias = torch.from_numpy(np.random.default_rng(m).normal(0, 0.1, n).astype(np.float32))
     lin = ttq.QuantLinear(ctx, fmt, torch.from_numpy(blocks), k, bias=bias.cuda())
     xd = x.cuda()
+    before = ctx.launch_count
     y = lin.forward(xd, out_dtype=torch.float32)
+    assert ctx.launch_count - before == 2
     again = lin.forward(xd, out_dtype=torch.float32)
     ctx.check_device_status()
     want = oracle.linear(OFMT[fmt], blocks, x_bits(x), odt(dtype), bias.numpy())
