@@ -618,7 +618,10 @@ def _linear_kernel_name(m: int) -> str:
         return "xprep_kernel + gemv_kernel<Q4_K> (activation planes bulk-copied from scratch)"
     if m <= 16:
         return "q4k_decode_kernel (one launch, integer-exact fp16 mma.sync)"
-    return "xh_prep_kernel + gemm_q4k_kernel / gemm_q4k_pair_kernel (tcgen05, tensor memory)"
+    if m <= 192:
+        return "xh_prep_kernel + gemm_ts_kernel (tcgen05, weights expanded into tensor memory)"
+    ts = ", gemm_ts_kernel for narrow matrices" if m <= 256 else ""
+    return f"xh_prep_kernel + gemm_q4k_kernel / gemm_q4k_pair_kernel (tcgen05, weights expanded into shared memory{ts})"
 
 
 def _time_graph(step, reps: int = 4, warm: int = 2) -> float:

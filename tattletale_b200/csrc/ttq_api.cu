@@ -646,7 +646,7 @@ static ttq_status linear_forward_impl(ttq_ctx *ctx, const ttq_weight *w, const v
     }
     // Q8_0 / Q6_K, 5 to 8 rows: the integer decode kernel keeps four rows' planes in shared memory and reads those of a second pass
     // from L2, row by row of weights; the exact form of the tensor-memory kernel does not care how many rows there are (4096 ->
-    // 28672, us: Q8_0 44 against 77, Q6_K 55 against 95; 4096 -> 128256 Q6_K 203 against 355).  From four items of 128 x 256
+    // 28672, us: Q8_0 45.6 against 77, Q6_K 56 against 95; 4096 -> 128256 Q6_K 206 against 355).  From four items of 128 x 256
     // weights per SM: below, its fixed cost does not pay (4096 -> 4096: 15.6 against 14.8 and 17.6 against 18.0).
     if (M >= 5 && M <= 8 && !gated && use_gemm && gemm_supported(w->fmt) && w->fmt != TTQ_FMT_Q4_K &&
         (w->N + 127) / 128 * w->SBp >= 4 * (int64_t)ctx->sms) {

@@ -3,8 +3,8 @@
 //
 // Operand roles.  The 128 rows (tensor-memory lanes) of the MMA are 128 ACTIVATION rows; its N dimension is the
 // CTA's 128 * NSUB expanded weight rows, so an epilogue thread owns one output row and stores runs of 16
-// consecutive features.  A row tile of BM = 64, 128 or 256 (grouped mode also 384) activation rows is MH = BM / 128
-// row blocks that share one expanded weight stage.
+// consecutive features.  A row tile of BM = 256 activation rows (plain and grouped mode also 64 and 128, grouped 384) is MH =
+// BM / 128 row blocks that share one expanded weight stage.
 //
 // Persistent CTAs (one per SM) walk output tiles of (128 * NSUB weight rows) x (BM activation rows); K may be cut
 // into `splits` work units whose fp32 partials a small kernel sums when the tiles alone cannot fill the SMs.
@@ -20,7 +20,7 @@
 //                weight tile.  Lane 0 of the first of them also brings the activation tile in with a single bulk
 //                async copy per stage (xh_prep_kernel stores fp16 activations as ready-made swizzled tile images).
 //                In the plain mode (weights already expanded to fp16 images by another kernel) these warps idle
-//                except for one producer lane that bulk-copies both operands.
+//                except for one producer warp that bulk-copies both operands (one elected lane).
 //   warp 20      allocates tensor memory, issues the MMAs (one elected lane) and commits them to the stage
 //                barriers.
 // A stage is one window of one 256-weight super-block: 64 K values (8 from each sub-block), in the order the
@@ -1202,7 +1202,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restr
                                                             const void *bias, int bias_dt, void *y, int y_dt, int64_t ldy) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const uint32_t n4 = (uint32_t)((N + 3) / 4), total = (uint32_t)M * n4;  // (a slab has at most 64 MB of activations: M * N / 4 fits)
+    const uint32_t n4 = (uint32_t)((N + 3) / 4), total = (uint32_t)M * n4;  // (the partial sums, splits * Mp * N floats, fit the 64 MB scratch)
     const bool vec = (N & 3) == 0;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < total; b += gridDim.x * blockDim.x) {
         const uint32_t m = b / n4;

@@ -20,13 +20,13 @@
 // 1700 cycles per SM, twice the HBM time of its 18 KB; from about 100 rows the activation slices (nb x 512 bytes per item out
 // of L2) and from 192 the tensor cores.  A fixed 9 us per linear go to the launch, the first tiles' latency and the sum of the
 // pieces.  Measured (4096 -> 28672 / 14336 -> 4096 / 4096 -> 6144 / 4096 -> 4096, us; the shared-memory GEMM in brackets):
-// 17 rows 30.4 / 20.3 / 13.2 / 11.8 (65.3 / 41.8 / 27.0 / 18.9), 64 rows 35.4 / 27.6 / 16.2 / 15.1 (65.6 / 42.9 / 30.0 / 20.0), 128 rows 50.7 / 36.8 / 23.1 / 21.7
-// (68.9 / 45.9 / 34.4 / 22.7); Q8_0 and Q6_K, 4096 -> 28672, 12 rows: 31.7 (69.5) and 38.3 (78.2).
+// 17 rows 30.7 / 20.0 / 12.8 / 11.3 (65.3 / 41.8 / 27.0 / 18.9), 64 rows 35.0 / 26.4 / 15.6 / 14.2 (65.6 / 42.9 / 30.0 / 20.0), 137 rows 56.0 / 37.6 / 23.2 / 21.0
+// (128 rows: 68.9 / 45.9 / 34.4 / 22.7); Q8_0 and Q6_K, 4096 -> 28672, 12 rows: 31.7 (69.5) and 38.3 (78.2).
 //
 // Exact form (Q8_0, Q6_K, one block of 16 rows): every weight as its fp16 rounding plus the remainder, two products into the same
 // accumulator, activations exact after a power of two per row, weights beyond fp16 brought into it by a power of two
-// per weight row (ts_row_power); half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 44 us,
-// Q6_K 55 (integer decode kernel: 77 and 95); error against 64 bits as the integer kernel's or below.
+// per weight row (ts_row_power); half an item per A stage.  4096 -> 28672, 5 to 8 rows: Q8_0 45.6
+// us, Q6_K 56 (integer decode kernel: 77 and 95); error against 64 bits as the integer kernel's or below.
 #include <cmath>
 
 #include "ttq_devutil.cuh"
