@@ -22,6 +22,7 @@
  *    on the GPU (two streams; the host entry points run on the context's own) must not be of the same kind:
  *      a  Q4_K up to 2 rows, Q8_0 / Q6_K up to 8, ttq_add_rmsnorm_prepare and ttq_linear_forward_prepared
  *      b  Q4_K of 3 to 16 rows (2 where K >= 8192); ttq_linear_forward_allreduce is of kinds a and b
+ *         (rows too long for that kernel are of kind c instead: count 3 to 16 rows as both unless K is small)
  *      c  Q4_K from 17 rows, Q8_0 / Q6_K from 9, trellis from 65        d  every trellis call        e  ttq_decode_attention
  *    An expert layer (ttq_moe) has a workspace of its own and overlaps with anything but itself.
  *  - Device-pointer entry points are asynchronous on `stream`; *_host entry points copy in, run,
