@@ -96,14 +96,15 @@ __global__ void __launch_bounds__(256) route_scatter_ordered_kernel(const int *_
     __shared__ int warp_count[8];
     const int e = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int base = row_start[e];
-    for (int64_t i0 = 0; i0 < pairs; i0 += 1024) {
-        const int64_t i = i0 + 4 * threadIdx.x;
+    const unsigned n = (unsigned)pairs;  // fewer than 2^30: 32-bit division (12000 pairs of 128 experts 12.7 -> 11.5 us; 3.9 with atomics)
+    for (unsigned i0 = 0; i0 < n; i0 += 1024) {
+        const unsigned i = i0 + 4 * threadIdx.x;
         int id[4], count = 0;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            id[q] = i + q < pairs ? ids[i + q] : -1;
+            id[q] = i + q < n ? ids[i + q] : -1;
             count += id[q] == e ? 1 : 0;
-            if (e == 0 && i + q < pairs && (id[q] < 0 || id[q] >= E)) slot_of[i + q] = -1;
+            if (e == 0 && i + q < n && (id[q] < 0 || id[q] >= E)) slot_of[i + q] = -1;
         }
         int upto = count;  // of the warp's threads up to this one
 #pragma unroll
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(256) route_scatter_ordered_kernel(const int *_
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (id[q] != e) continue;
-            if (slot < Mp) row_src[slot] = (int)((i + q) / top_k);
+            if (slot < Mp) row_src[slot] = (int)((i + q) / (unsigned)top_k);
             slot_of[i + q] = slot < Mp ? slot : -1;
             slot++;
         }
